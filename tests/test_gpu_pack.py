@@ -121,3 +121,26 @@ def test_dequant_crafted_edge_cases():
     got = quant.dequant(torch.from_numpy(qweight.view(np.int32)).cuda(),
                         torch.from_numpy(zs.view(np.float16)).cuda(), N, K, g)
     assert np.array_equal(got.cpu().numpy().view(np.uint16), expect.view(np.uint16))
+
+
+@pytest.mark.parametrize("N,K,g,shift", [(32, 32, 32, 0), (64, 160, 32, 4), (96, 192, 64, 4), (32, 384, 128, 0), (64, 256, 128, 4)])
+def test_fused_quantize_pack_edges(N, K, g, shift):
+    """Blocks narrower than the 128 in-features a CTA takes, groups whose values lie far from zero compared with their
+    spread (min / scale beyond every clamp), and a weight that starts on an 8-byte boundary only (`shift` halfs into its
+    buffer: the kernel's half-vector variant): bit-identical to the oracle."""
+    import quant
+    gen = torch.Generator().manual_seed(N + K + shift)
+    w = (torch.randn(N, K, generator=gen) * 0.02).half()
+    w[1] = (100.0 + torch.rand(K, generator=gen) * 0.2).half()
+    w[2] = (-900.0 + torch.rand(K, generator=gen)).half()
+    w[3] = (torch.randn(K, generator=gen) * 1e-6).half()
+    qw8, zeros, scales, w_fp16 = oracle.generate_quant(w, 4, g)
+    o_qw, o_zs = oracle.pack(qw8, zeros, scales, K, N, g)
+    buf = torch.empty(N * K + shift, dtype=torch.float16, device="cuda")
+    d = buf[shift:].view(N, K)
+    d.copy_(w)
+    qw, zs, d_wfp16, ours, _, d_scales = quant.quantize_pack(d, K, N, g, parts=True)
+    assert torch.equal(ours.cpu(), qw8)
+    assert np.array_equal(d_scales.cpu().numpy().view(np.uint16), scales.numpy().view(np.uint16))
+    assert np.array_equal(d_wfp16.cpu().numpy().view(np.uint16), w_fp16.numpy().view(np.uint16))
+    assert np.array_equal(qw.cpu().numpy().view(np.uint32), o_qw) and np.array_equal(zs.cpu().numpy().view(np.uint16), o_zs)
