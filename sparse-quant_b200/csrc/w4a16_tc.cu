@@ -8,8 +8,8 @@
 // out-features per CTA tile), the activations are "B" (N = 64/128/256 tokens), the fp32
 // accumulator D[out-feature lane][token column] lives in tensor memory.
 //
-// One persistent CTA per SM, warp specialised (warp numbers: 0-3 and 6.. dequantisers, 4 and the last one TMA, 5 MMA;
-// 352 threads with the 256-token tile, 608 with the smaller ones, which have two more dequantiser groups).
+// One persistent CTA of 608 threads per SM, warp specialised (warp 4 and the last one TMA, 5 MMA, sixteen workers:
+// dequantisers and, with the 256-token tile, epilogue warps).
 //
 // What set the pace of earlier versions was the ISSUE cost of the tensor-core instructions in the one thread that may
 // issue them (measured on B200 with a loop of nothing but MMAs, 148 CTAs): from a loop that a single lane enters a
@@ -33,7 +33,7 @@
 //   W ring   (shared memory, own depth): the stage's packed weight tiles (a k-tile row of the format is contiguous:
 //            plain bulk copies) and the (zero, scale) row(s), filled by the last warp, read only by the dequantisers and
 //            released as soon as they hold the words in registers.
-//   warps0-3,6.. dequantisers (groups of four; a pair of groups takes the two 64-k halves of a stage; with the 64- and
+//   dequantisers (groups of four; a pair of groups takes the two 64-k halves of a stage; with the 64- and
 //            128-token tiles, whose stages are shorter than a pair's latency chain, two pairs take stages in turn -
 //            measured 3-7 % there): read 16 B per lane per 32x32 tile from shared memory, expand the nibbles in
 //            registers, (t - z) * s with
@@ -43,8 +43,9 @@
 //   warp 5   MMA issuer: tcgen05.mma kind::f16 with A from tensor memory and B from the swizzled shared-memory
 //            tile, eight K=16 instructions and two commits per stage; the barriers needed next are probed before
 //            the MMAs in front of them are issued, so that in steady state no barrier round trip sits between them.
-//   warps0-3,6-9 epilogue (the first pair of groups, after their last dequant step of the tile): tcgen05.ld the accumulator,
-//            fp32 -> fp16, bias add, transposed store to out[token, out-feature].
+//   epilogue (two groups of workers: 10-17 with the 256-token tile, else the first pair after their last dequant step of
+//            the tile): tcgen05.ld the accumulator, fp32 -> fp16, release it, bias add, transposed store to
+//            out[token, out-feature].
 // No cluster fan-out is used anywhere.  Every mbarrier wait is bounded; on a timeout the CTA raises an error word
 // in global memory, drains and frees its tensor memory, and returns.
 #include <mutex>
@@ -63,15 +64,14 @@ namespace {
 constexpr int kBlockN   = 128;                 // out-features per CTA tile (4 packed tiles)
 constexpr int kBlockK   = 128;                 // k per pipeline stage (4 packed tiles, eight MMAs, one commit)
 constexpr int kSubK     = 64;                  // k per swizzled activation sub-tile (128 bytes of fp16)
-// GROUPS = groups of four dequantiser warps: 2 (one per 64-k half of every stage) for the 256-token tile, 4 (two
-// pairs taking stages in turn) for the smaller tiles, whose stages are shorter than one pair's latency chain.
-// Warps 0-3, 6.. : dequantisers; 4: x TMA; 5: MMA; the last warp: W TMA.
-__host__ __device__ constexpr int w_producer_warp(int groups) { return 2 + 4 * groups; }
-__host__ __device__ constexpr int tc_threads(int groups) { return 32 * (w_producer_warp(groups) + 1); }
-#ifndef W4A16_TC_GROUPS_SMALL
-#define W4A16_TC_GROUPS_SMALL 4
-#endif
-__host__ __device__ constexpr int tc_groups(int tok) { return tok == 256 ? 2 : W4A16_TC_GROUPS_SMALL; }
+// Warps 4: x TMA; 5: MMA; the last one: W TMA; the other sixteen are workers in groups of four (0-3, 6-9, 10-13, 14-17).
+// Dequantiser groups: with the 256-token tile the first two (one per 64-k half of every stage), the other two being
+// epilogue warps; with the smaller tiles, whose stages are shorter than one pair's latency chain, all four (two pairs
+// taking stages in turn), the first pair draining the accumulator as well.
+constexpr int kWorkerGroups = 4;
+constexpr int kWProducerWarp = 2 + 4 * kWorkerGroups;
+constexpr int kTcThreads = 32 * (kWProducerWarp + 1);
+__host__ __device__ constexpr int tc_groups(int tok) { return tok == 256 ? 2 : 4; }
 constexpr int kTmemCols = 512;
 constexpr uint64_t kWaitBudgetNs = 400ull * 1000 * 1000;   // 0.4 s: far above any legitimate wait
 
@@ -91,7 +91,7 @@ struct TcCfg {
     static constexpr int kBarriers = 5 * kStages + 2 * kWStages + 3;
     static_assert(8 * kBarriers + 12 <= kBarrierBytes, "barrier area");
     static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
-    static_assert(kACol + 64 * kStages <= kTmemCols, "TMEM budget");
+    static_assert(kACol + 64 * kStages + (TOK == 256 ? 64 : 0) <= kTmemCols, "TMEM budget");
 };
 
 struct TcParams {
@@ -110,8 +110,17 @@ struct TcParams {
     long long* account;             // debug builds: cycle accounting of CTA 0's MMA warp (8 words), or null
 };
 
+// Two fp32 bit patterns -> half2, round to nearest even.  Volatile: stays between the tensor memory loads around it, or
+// the compiler keeps the 128 fp32 values of a thread until all are loaded.
+__device__ __forceinline__ uint32_t pack_halves(uint32_t lo, uint32_t hi)
+{
+    uint32_t r;
+    asm volatile("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(__uint_as_float(hi)), "f"(__uint_as_float(lo)));
+    return r;
+}
+
 template <int TOK>
-__global__ void __launch_bounds__(tc_threads(tc_groups(TOK)), 1) tc_kernel(const __grid_constant__ CUtensorMap x_map, const TcParams p)
+__global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant__ CUtensorMap x_map, const TcParams p)
 {
     using Cfg = TcCfg<TOK>;
     constexpr int S = Cfg::kStages, SW = Cfg::kWStages;
@@ -201,7 +210,7 @@ __global__ void __launch_bounds__(tc_threads(tc_groups(TOK)), 1) tc_kernel(const
             }
             if (!ok) drain_copies();
         }
-    } else if (warp == w_producer_warp(tc_groups(TOK))) {
+    } else if (warp == kWProducerWarp) {
         // ------------------------------ TMA producer of the packed weights ------------------------------
         // Three lanes share the copies of a stage (an issued copy holds its thread for about a hundred cycles).  A
         // copy that completes before lane 0 has armed the barrier only drives its byte count negative for a moment;
@@ -344,19 +353,21 @@ __global__ void __launch_bounds__(tc_threads(tc_groups(TOK)), 1) tc_kernel(const
         }
 #endif
     } else {
-        // ------------------------------ dequant + epilogue (warps 0..3 and 6..9) ------------------------------
-        // Two groups of four warps; a warp may only touch the TMEM lane quarter (warp index % 4), which is also the
+        // ------------------------------ dequant + epilogue (the worker warps) ------------------------------
+        // Groups of four warps; a warp may only touch the TMEM lane quarter (warp index % 4), which is also the
         // packed tile column it dequantises.  Group g takes the g-th 64-k half of every stage: a half keeps a warp
         // busy for a chain of dependent latencies (shared-memory load, unpack, sub/mul, tcgen05.st, its completion),
-        // which the ring depth covers.  Both groups also drain the accumulator (half of the columns each) in the
-        // epilogue.
+        // which the ring depth covers.  Two groups drain the accumulator (half of the columns each): with the
+        // 256-token tile groups of their own, so that the dequantisers run on into the next tile (its first stages are
+        // ready when the accumulator is free again), otherwise the first pair.
         int st = 0, sw = 0; uint32_t phase = 0, wphase = 0, dphase = 0;
         bool ok = true;
         const int r = lane >> 2;
         constexpr int GROUPS = tc_groups(TOK);
+        constexpr bool kOwnEpilogue = GROUPS < kWorkerGroups;
         const int quarter = warp & 3;
-        const int wgroup = warp < 4 ? 0 : (warp - 2) / 4;              // 0 .. GROUPS-1
-        const int dgroup = wgroup & 1;                                 // which 64-k half of a stage
+        const int wgroup = warp < 4 ? 0 : (warp - 2) / 4;              // 0 .. kWorkerGroups-1
+        const int dgroup = wgroup & 1;                                 // which 64-k half of a stage / half of the accumulator's columns
         const int turn = wgroup >> 1;                                  // GROUPS == 4: which stages (even / odd)
         uint32_t step_mod = 0;
         uint32_t epi_phase = 0;
@@ -370,9 +381,175 @@ __global__ void __launch_bounds__(tc_threads(tc_groups(TOK)), 1) tc_kernel(const
         };
         const uint32_t lane_field = (uint32_t)(quarter * 32) << 16;
         const int zs_row = p.g == 64 ? dgroup : 0;                     // (zero, scale) row of this group's half
-        for (int item = blockIdx.x; item < total_tiles && ok; item += gridDim.x) {
+        // the epilogue of one work item: drains the accumulator (half of the columns per group), false = a wait gave up
+        auto epilogue = [&](int item) -> bool {
             const int tile = item / p.split, kp = item % p.split;
             const int nb = tile % p.n_blocks, tb = tile / p.n_blocks;
+            // epilogue: thread = out-feature (TMEM lane), registers = tokens.  A warp's columns are rounded to fp16 and
+            // the accumulator is released before bias / ReLU / residual / stores (whose loops carry no test per element:
+            // with the tests inside a tile took 15 000 cycles to drain, without them 5 000), so that the MMA of the next
+            // tile waits for the tensor memory reads alone.  A missing bias is added as -0.0, which changes no value.
+            // Measured with the 256-token tile, whose dequantisers used to drain it themselves: 8192 tokens x 16384 -> 4096
+            // with residual 1148 -> 886 us (1240 TFLOP/s), 2048 x 4096 -> 16384 with ReLU 255 -> 226 us, same results.
+            if (!__all_sync(0xffffffffu, mbar_wait(dfull_bar, dphase, abort_flag, kWaitBudgetNs))) return false;
+            dphase ^= 1u;
+            tc_fence_after_sync();
+            const int n = nb * kBlockN + quarter * 32 + lane;
+            const bool n_ok = n < p.N;
+            const __half bias = (p.bias && n_ok) ? p.bias[n] : __ushort_as_half((unsigned short)0x8000u);
+            const int tok0 = tb * TOK;
+            const bool full_tile = tok0 + TOK <= p.tokens;
+            constexpr int kCols = TOK / 2;                                       // columns (tokens) of this warp
+            const int c_begin = dgroup * kCols, c_end = c_begin + kCols;
+            auto release_accumulator = [&]() {
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(dempty_bar);
+            };
+            if (p.split == 1) {
+                // 64 columns make 32 packed registers; the other half of a 256-token tile's columns is parked, packed, in
+                // the tensor memory columns that neither the accumulator nor the A ring uses
+                constexpr int kPass = kCols < 64 ? kCols : 64;
+                uint32_t h[kPass / 2];                                           // fp16 pairs: tokens 2i, 2i + 1 of the pass
+                auto fetch = [&](int col) {
+#pragma unroll
+                    for (int c = 0; c < kPass; c += 16) {
+                        uint32_t v[16];
+                        tmem_ld_32x32b_x16(tmem_base + lane_field + col + c, v);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) h[c / 2 + j] = pack_halves(v[2 * j], v[2 * j + 1]);
+                    }
+                };
+                const __half2 bias2 = __half2half2(bias);
+                auto emit = [&](int col) {
+                    const int live = min(p.tokens - tok0 - col, kPass);          // rows of this pass that exist
+                    const size_t at = (size_t)(tok0 + col) * p.N + n;
+                    __half* dst = p.out + at;
+                    const __half* res = p.residual + at;
+#pragma unroll
+                    for (int i = 0; i < kPass / 2; i += 4) {                     // eight tokens at a time
+                        __half2 o[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) o[j] = __hadd2(*reinterpret_cast<__half2*>(&h[i + j]), bias2);
+                        if (p.relu) {
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) o[j] = __hmax2(o[j], __half2half2(__half()));
+                        }
+                        if (p.residual) {
+                            __half r[8];
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) r[j] = 2 * i + j < live ? res[(size_t)(2 * i + j) * p.N] : __half();
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) o[j] = __hadd2(o[j], __halves2half2(r[2 * j], r[2 * j + 1]));
+                        }
+                        if (2 * i + 8 <= live) {
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                dst[(size_t)(2 * (i + j)) * p.N] = __low2half(o[j]);
+                                dst[(size_t)(2 * (i + j) + 1) * p.N] = __high2half(o[j]);
+                            }
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                                if (2 * i + j < live) dst[(size_t)(2 * i + j) * p.N] = (j & 1) ? __high2half(o[j / 2]) : __low2half(o[j / 2]);
+                        }
+                    }
+                };
+                const uint32_t park = tmem_base + lane_field + Cfg::kACol + 64 * S + 32 * dgroup;
+                fetch(c_begin);
+                if constexpr (kCols > kPass) {
+                    tmem_st_32x32b_x32(park, h);
+                    fetch(c_begin + kPass);
+                    tmem_wait_st();
+                }
+                release_accumulator();
+                if (n_ok) emit(c_end - kPass);
+                if constexpr (kCols > kPass) {
+                    __syncwarp();
+                    tmem_ld_32x32b_x32(park, h);
+                    tmem_wait_ld();
+                    if (n_ok) emit(c_begin);
+                }
+                return true;
+            }
+            auto finish = [&](float acc, int t) {                                // one output element
+                __half h = __hadd(__float2half_rn(acc), bias);
+                if (p.relu) h = __hmax(h, __half());
+                if (p.residual) h = __hadd(h, p.residual[(size_t)t * p.N + n]);
+                p.out[(size_t)t * p.N + n] = h;
+            };
+            const bool plain = full_tile && !p.relu && !p.residual;
+            // split-K: park the fp32 partial tile in the workspace; the CTA that completes the tile (the last
+            // of `split` arrivals, found with one atomic per CTA) adds the parts in a fixed order - deterministic.
+            float* mine = p.partial + (size_t)kp * p.tokens * p.N;
+#pragma unroll 1
+            for (int c0 = c_begin; c0 < c_end; c0 += 32) {
+                uint32_t v[32];
+                tmem_ld_32x32b_x32(tmem_base + lane_field + c0, v);
+                tmem_wait_ld();
+                if (c0 + 32 >= c_end) release_accumulator();
+                if (!n_ok) continue;
+                float* dst = mine + (size_t)(tok0 + c0) * p.N + n;
+                if (full_tile) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) dst[(size_t)j * p.N] = __uint_as_float(v[j]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        if (tok0 + c0 + j < p.tokens) dst[(size_t)j * p.N] = __uint_as_float(v[j]);
+                }
+            }
+            __threadfence();
+            if (!epi_sync()) return false;                              // every warp's part of the tile is in the workspace
+            if (wgroup == (kOwnEpilogue ? GROUPS : 0) && quarter == (kOwnEpilogue ? 2 : 0) && lane == 0) {     // one thread of the draining groups
+                const int old = atomicAdd(p.counters + tile, 1);
+                const int last = old == p.split - 1;
+                if (last) p.counters[tile] = 0;                          // ready for the next launch
+                *last_flag = last;
+            }
+            if (!epi_sync()) return false;
+            if (*last_flag) {
+                __threadfence();
+                if (n_ok) {
+                    // 32 tokens per batch: part 0, then one part at a time added to it (fixed order, up to 32
+                    // loads in flight per thread - the reduction is a chain of L2 round trips otherwise)
+                    const int c_last = min(c_end, p.tokens - tok0);      // ragged tile: stop at the last token
+#pragma unroll 1
+                    for (int c = c_begin; c < c_last; c += 32) {
+                        const float* src = p.partial + (size_t)(tok0 + c) * p.N + n;
+                        const bool whole = c + 32 <= c_last;
+                        float sum[32];
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) sum[j] = (whole || c + j < c_last) ? __ldcg(src + (size_t)j * p.N) : 0.f;
+                        for (int q = 1; q < p.split; ++q) {
+                            const float* sq = src + (size_t)q * p.tokens * p.N;
+                            float part[32];
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) part[j] = (whole || c + j < c_last) ? __ldcg(sq + (size_t)j * p.N) : 0.f;
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) sum[j] += part[j];
+                        }
+                        if (whole && plain) {
+                            __half* dst = p.out + (size_t)(tok0 + c) * p.N + n;
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) dst[(size_t)j * p.N] = __hadd(__float2half_rn(sum[j]), bias);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j)
+                                if (c + j < c_last) finish(sum[j], tok0 + c + j);
+                        }
+                    }
+                }
+            }
+            return epi_sync();                                               // last_flag may be rewritten by the next item
+        };
+        const int dequant_tiles = kOwnEpilogue && wgroup >= GROUPS ? 0 : total_tiles;
+        if (kOwnEpilogue && wgroup >= GROUPS) {
+            for (int item = blockIdx.x; item < total_tiles && ok; item += gridDim.x) ok = epilogue(item);
+        }
+        for (int item = blockIdx.x; item < dequant_tiles && ok; item += gridDim.x) {
+            const int nb = (item / p.split) % p.n_blocks;
             const bool has_tile = nb * 4 + quarter < n_tiles;
             int ks0, ks1;
             k_range(item, ks0, ks1);
@@ -431,119 +608,7 @@ __global__ void __launch_bounds__(tc_threads(tc_groups(TOK)), 1) tc_kernel(const
                 if (++st == S) { st = 0; phase ^= 1u; }
             }
             if (!ok) break;
-            if (wgroup >= 2) continue;                                       // only the first pair drains the accumulator
-
-            // epilogue: thread = out-feature (TMEM lane), registers = tokens.  The per-element loops carry no branch
-            // (measured: with the bias / ReLU / residual / ragged-tile tests inside them a tile took 15 000 cycles to
-            // drain, without them 5 000): the common case - full token tile, no ReLU, no residual - has its own loop,
-            // and a missing bias is added as -0.0, which changes no value.
-            ok = __all_sync(0xffffffffu, mbar_wait(dfull_bar, dphase, abort_flag, kWaitBudgetNs));
-            if (!ok) break;
-            dphase ^= 1u;
-            tc_fence_after_sync();
-            const int n = nb * kBlockN + quarter * 32 + lane;
-            const bool n_ok = n < p.N;
-            const __half bias = (p.bias && n_ok) ? p.bias[n] : __ushort_as_half((unsigned short)0x8000u);
-            const int tok0 = tb * TOK;
-            const bool full_tile = tok0 + TOK <= p.tokens;
-            const bool plain = full_tile && !p.relu && !p.residual;
-            const int c_begin = dgroup * (TOK / 2), c_end = (dgroup + 1) * (TOK / 2);
-            // the accumulator is free again once this warp's columns are in registers: the MMA of the next tile
-            // starts while the values are still being converted and stored
-            auto release_accumulator = [&]() {
-                tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(dempty_bar);
-            };
-            auto finish = [&](float acc, int t) {                                // general path: one output element
-                __half h = __hadd(__float2half_rn(acc), bias);
-                if (p.relu) h = __hmax(h, __half());
-                if (p.residual) h = __hadd(h, p.residual[(size_t)t * p.N + n]);
-                p.out[(size_t)t * p.N + n] = h;
-            };
-            if (p.split == 1) {
-#pragma unroll 1
-                for (int c0 = c_begin; c0 < c_end; c0 += 32) {
-                    uint32_t v[32];
-                    tmem_ld_32x32b_x32(tmem_base + lane_field + c0, v);
-                    tmem_wait_ld();
-                    if (c0 + 32 >= c_end) release_accumulator();
-                    if (!n_ok) continue;
-                    if (plain) {
-                        __half* dst = p.out + (size_t)(tok0 + c0) * p.N + n;
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) dst[(size_t)j * p.N] = __hadd(__float2half_rn(__uint_as_float(v[j])), bias);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (tok0 + c0 + j < p.tokens) finish(__uint_as_float(v[j]), tok0 + c0 + j);
-                    }
-                }
-            } else {
-                // split-K: park the fp32 partial tile in the workspace; the CTA that completes the tile (the last
-                // of `split` arrivals, found with one atomic per CTA) adds the parts in a fixed order - deterministic.
-                float* mine = p.partial + (size_t)kp * p.tokens * p.N;
-#pragma unroll 1
-                for (int c0 = c_begin; c0 < c_end; c0 += 32) {
-                    uint32_t v[32];
-                    tmem_ld_32x32b_x32(tmem_base + lane_field + c0, v);
-                    tmem_wait_ld();
-                    if (c0 + 32 >= c_end) release_accumulator();
-                    if (!n_ok) continue;
-                    float* dst = mine + (size_t)(tok0 + c0) * p.N + n;
-                    if (full_tile) {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) dst[(size_t)j * p.N] = __uint_as_float(v[j]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (tok0 + c0 + j < p.tokens) dst[(size_t)j * p.N] = __uint_as_float(v[j]);
-                    }
-                }
-                __threadfence();
-                if (!(ok = epi_sync())) break;                               // every warp's part of the tile is in the workspace
-                if (warp == 0 && lane == 0) {
-                    const int old = atomicAdd(p.counters + tile, 1);
-                    const int last = old == p.split - 1;
-                    if (last) p.counters[tile] = 0;                          // ready for the next launch
-                    *last_flag = last;
-                }
-                if (!(ok = epi_sync())) break;
-                if (*last_flag) {
-                    __threadfence();
-                    if (n_ok) {
-                        // 32 tokens per batch: part 0, then one part at a time added to it (fixed order, up to 32
-                        // loads in flight per thread - the reduction is a chain of L2 round trips otherwise)
-                        const int c_last = min(c_end, p.tokens - tok0);      // ragged tile: stop at the last token
-#pragma unroll 1
-                        for (int c = c_begin; c < c_last; c += 32) {
-                            const float* src = p.partial + (size_t)(tok0 + c) * p.N + n;
-                            const bool whole = c + 32 <= c_last;
-                            float sum[32];
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) sum[j] = (whole || c + j < c_last) ? __ldcg(src + (size_t)j * p.N) : 0.f;
-                            for (int q = 1; q < p.split; ++q) {
-                                const float* sq = src + (size_t)q * p.tokens * p.N;
-                                float part[32];
-#pragma unroll
-                                for (int j = 0; j < 32; ++j) part[j] = (whole || c + j < c_last) ? __ldcg(sq + (size_t)j * p.N) : 0.f;
-#pragma unroll
-                                for (int j = 0; j < 32; ++j) sum[j] += part[j];
-                            }
-                            if (whole && plain) {
-                                __half* dst = p.out + (size_t)(tok0 + c) * p.N + n;
-#pragma unroll
-                                for (int j = 0; j < 32; ++j) dst[(size_t)j * p.N] = __hadd(__float2half_rn(sum[j]), bias);
-                            } else {
-#pragma unroll
-                                for (int j = 0; j < 32; ++j)
-                                    if (c + j < c_last) finish(sum[j], tok0 + c + j);
-                            }
-                        }
-                    }
-                }
-                if (!(ok = epi_sync())) break;                               // last_flag may be rewritten by the next item
-            }
+            if (!kOwnEpilogue && wgroup < 2) ok = epilogue(item);            // the first pair drains the accumulator
         }
     }
 
@@ -645,7 +710,7 @@ int launch_tok(const CUtensorMap& map, const TcParams& p, int grid, cudaStream_t
         if (e != cudaSuccess) return record_cuda_error(e);
         if (dev < 64) configured[dev] = 1;
     }
-    tc_kernel<TOK><<<grid, tc_threads(tc_groups(TOK)), TcCfg<TOK>::kSmemBytes, st>>>(map, p);
+    tc_kernel<TOK><<<grid, kTcThreads, TcCfg<TOK>::kSmemBytes, st>>>(map, p);
     count_launch();
     e = cudaGetLastError();
     return e == cudaSuccess ? W4A16_OK : record_cuda_error(e);
