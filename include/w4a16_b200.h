@@ -245,6 +245,16 @@ int w4a16_gemm_allreduce_residual(const void* x, const void* qweight, const void
 int w4a16_decode_attention(const void* qkv, void* k_cache, void* v_cache, void* out, const void* pos,
                            const void* rope_cos, const void* rope_sin, int batch, int heads, int head_dim,
                            int max_len, int qkv_stride, float scale, void* stream);
+/*
+ * What a prompt's q/k/v projection output goes through on its way to attention, in one launch: the rotary embedding on
+ * q (in place) and k, and the new keys and values appended to the static cache.
+ *   qkv      fp16 [batch, seq, qkv_stride], row = [q (heads*head_dim) | k | v]; 16-byte aligned, qkv_stride % 8 == 0
+ *   k_cache, v_cache  fp16 [batch, heads, max_len, head_dim], 16-byte aligned; rows pos0 .. pos0+seq-1 are written
+ *   rope_cos, rope_sin  fp16 [>= seq, head_dim] tables of the positions pos0 .. or both NULL (q is then left alone)
+ * head_dim % 16 == 0.  The rotation is computed in fp32 and rounded to fp16 once.
+ */
+int w4a16_append_qkv(void* qkv, void* k_cache, void* v_cache, const void* rope_cos, const void* rope_sin, int batch,
+                     int seq, int heads, int head_dim, int max_len, int pos0, int qkv_stride, void* stream);
 /* Tuning hook (tests, benchmarks): CTAs per (head, sequence) splitting the cached positions, 0 = automatic. */
 void w4a16_tune_attention(int split);
 /* Tuning hook: 1 launches the small decode-step kernels with programmatic stream serialization, 0 (default) in plain
@@ -268,6 +278,9 @@ int w4a16_add_norm(const void* x, const void* delta, void* x_out, void* h_out, c
  * (act_fn(gate_proj(x)) * up_proj(x), modeling_llama_ours.py:272) on the output [rows, 2n] of the gate/up projections
  * fused into one GEMV; fp16, n % 8 == 0. */
 int w4a16_silu_mul(const void* gate_up, void* out, int rows, int n, void* stream);
+/* The same product on the output of a linear whose 32-wide gate and up tiles alternate (the layout W4A16_FLAG_SILU_MUL
+ * asks for): gate_up fp16 [rows, 2n] = g0 u0 g1 u1 ..., out fp16 [rows, n]; n % 32 == 0. */
+int w4a16_silu_mul_tiles(const void* gate_up, void* out, int rows, int n, void* stream);
 
 /*
  * Normalisation folded into the decode GEMV that consumes it, residual add into the GEMV that produces the block

@@ -236,6 +236,68 @@ __global__ void __launch_bounds__(kAttnThreads) decode_attention_kernel(const At
     cluster.sync();                                                         // rank 0 may still be reading this CTA's part[]
 }
 
+// ---- prompts: rotary embedding of q (in place) and k, keys and values into the cache ----
+struct AppendParams {
+    __half* qkv;
+    __half* k_cache;
+    __half* v_cache;
+    const __half* rope_cos;
+    const __half* rope_sin;
+    int seq, heads, head_dim, max_len, pos0, qkv_stride;
+    unsigned lanes;          // head_dim / 16: threads of one (row, head)
+    unsigned total;          // batch * seq * heads * lanes
+};
+
+// A thread owns dims 8j .. 8j+7 of one (row, head) and their partners head_dim/2 further on, so that "rotate half" stays
+// inside it.  Bound: memory, one pass (read k, v, with rotation q; write the same).  4096 tokens x 4096 without rotation:
+// 21 us (6.3 TB/s) for the two strided torch copies of 43 us each that it replaces.
+__device__ __forceinline__ void rotate8(uint4& lo, uint4& hi, const uint4& cl, const uint4& ch, const uint4& sl, const uint4& sh)
+{
+    __half2* a = reinterpret_cast<__half2*>(&lo);
+    __half2* b = reinterpret_cast<__half2*>(&hi);
+    const __half2* c0 = reinterpret_cast<const __half2*>(&cl);
+    const __half2* c1 = reinterpret_cast<const __half2*>(&ch);
+    const __half2* s0 = reinterpret_cast<const __half2*>(&sl);
+    const __half2* s1 = reinterpret_cast<const __half2*>(&sh);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float2 x = __half22float2(a[e]), y = __half22float2(b[e]);
+        const float2 cx = __half22float2(c0[e]), cy = __half22float2(c1[e]), sx = __half22float2(s0[e]), sy = __half22float2(s1[e]);
+        a[e] = __floats2half2_rn(x.x * cx.x - y.x * sx.x, x.y * cx.y - y.y * sx.y);      // x cos + rotate_half(x) sin
+        b[e] = __floats2half2_rn(y.x * cy.x + x.x * sy.x, y.y * cy.y + x.y * sy.y);
+    }
+}
+
+__global__ void __launch_bounds__(256) append_qkv_kernel(const AppendParams p)
+{
+    const unsigned i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= p.total) return;
+    const unsigned j = i % p.lanes, rh = i / p.lanes;
+    const unsigned head = rh % (unsigned)p.heads, row = rh / (unsigned)p.heads;
+    const unsigned b = row / (unsigned)p.seq, s = row - b * (unsigned)p.seq;
+    const int D = p.head_dim, half = D / 2;
+    __half* q = p.qkv + (size_t)row * p.qkv_stride + head * D + 8 * j;
+    const __half* k = q + p.heads * D;
+    const __half* v = k + p.heads * D;
+    const size_t at = (((size_t)b * p.heads + head) * p.max_len + p.pos0 + s) * D + 8 * j;
+    uint4 k0 = *reinterpret_cast<const uint4*>(k), k1 = *reinterpret_cast<const uint4*>(k + half);
+    const uint4 v0 = *reinterpret_cast<const uint4*>(v), v1 = *reinterpret_cast<const uint4*>(v + half);
+    if (p.rope_cos) {
+        const size_t t = (size_t)s * D + 8 * j;
+        const uint4 cl = *reinterpret_cast<const uint4*>(p.rope_cos + t), ch = *reinterpret_cast<const uint4*>(p.rope_cos + t + half);
+        const uint4 sl = *reinterpret_cast<const uint4*>(p.rope_sin + t), sh = *reinterpret_cast<const uint4*>(p.rope_sin + t + half);
+        uint4 q0 = *reinterpret_cast<const uint4*>(q), q1 = *reinterpret_cast<const uint4*>(q + half);
+        rotate8(q0, q1, cl, ch, sl, sh);
+        rotate8(k0, k1, cl, ch, sl, sh);
+        *reinterpret_cast<uint4*>(q) = q0;
+        *reinterpret_cast<uint4*>(q + half) = q1;
+    }
+    *reinterpret_cast<uint4*>(p.k_cache + at) = k0;
+    *reinterpret_cast<uint4*>(p.k_cache + at + half) = k1;
+    *reinterpret_cast<uint4*>(p.v_cache + at) = v0;
+    *reinterpret_cast<uint4*>(p.v_cache + at + half) = v1;
+}
+
 int g_force_attn_split = 0;
 
 template <int D>
@@ -283,6 +345,27 @@ using namespace w4a16;
 
 // Tuning hook for tests and benchmarks: CTAs per (head, sequence), 0 = automatic.  Not part of the drop-in surface.
 extern "C" void w4a16_tune_attention(int split) { w4a16::g_force_attn_split = (split == 1 || split == 2 || split == 4 || split == 8) ? split : 0; }
+
+extern "C" int w4a16_append_qkv(void* qkv, void* k_cache, void* v_cache, const void* rope_cos, const void* rope_sin, int batch,
+                                int seq, int heads, int head_dim, int max_len, int pos0, int qkv_stride, void* stream)
+{
+    if (!qkv || !k_cache || !v_cache || ((rope_cos == nullptr) != (rope_sin == nullptr))) return W4A16_ERR_NULL_POINTER;
+    if (batch <= 0 || seq <= 0 || heads <= 0 || head_dim <= 0 || (head_dim % 16) || pos0 < 0 || max_len <= 0 ||
+        (long long)pos0 + seq > max_len || qkv_stride < 3ll * heads * head_dim || (qkv_stride % 8))
+        return W4A16_ERR_BAD_SHAPE;
+    if (((uintptr_t)qkv | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)rope_cos | (uintptr_t)rope_sin) & 15) return W4A16_ERR_MISALIGNED;
+    const long long total = (long long)batch * seq * heads * (head_dim / 16);
+    if (total >= (1ll << 31)) return W4A16_ERR_TOO_LARGE;
+    AppendParams p;
+    p.qkv = (__half*)qkv; p.k_cache = (__half*)k_cache; p.v_cache = (__half*)v_cache;
+    p.rope_cos = (const __half*)rope_cos; p.rope_sin = (const __half*)rope_sin;
+    p.seq = seq; p.heads = heads; p.head_dim = head_dim; p.max_len = max_len; p.pos0 = pos0; p.qkv_stride = qkv_stride;
+    p.lanes = (unsigned)(head_dim / 16); p.total = (unsigned)total;
+    append_qkv_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(p);
+    count_launch();
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? W4A16_OK : record_cuda_error(e);
+}
 
 extern "C" int w4a16_decode_attention(const void* qkv, void* k_cache, void* v_cache, void* out, const void* pos,
                                       const void* rope_cos, const void* rope_sin, int batch, int heads, int head_dim,

@@ -57,10 +57,12 @@ C_ABI = {
     "w4a16_gemm_allreduce_residual": (_ci, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _ci, _ci, _ci, _ci, _ci, ctypes.POINTER(_vp), _ci,
                                             _ci, _sz, _vp, ctypes.c_uint]),
     "w4a16_decode_attention": (_ci, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _ci, _ci, _ci, _ci, _ci, ctypes.c_float, _vp]),
+    "w4a16_append_qkv": (_ci, [_vp, _vp, _vp, _vp, _vp, _ci, _ci, _ci, _ci, _ci, _ci, _ci, _vp]),
     "w4a16_tune_attention": (None, [_ci]),
     "w4a16_tune_aux_launch": (None, [_ci]),
     "w4a16_add_norm": (_ci, [_vp, _vp, _vp, _vp, _vp, _vp, _ci, _ci, ctypes.c_float, _ci, _vp]),
     "w4a16_silu_mul": (_ci, [_vp, _vp, _ci, _ci, _vp]),
+    "w4a16_silu_mul_tiles": (_ci, [_vp, _vp, _ci, _ci, _vp]),
     "w4a16_gemm_static_scratch": (_ci, [_vp, _vp, _vp, _vp, _vp, _ci, _ci, _ci, _ci, _vp]),
     "w4a16_static_scratch_error_flag": (_ci, [ctypes.POINTER(_ci)]),
     "w4a16_dequant": (_ci, [_vp, _vp, _vp, _ci, _ci, _ci, _vp]),
@@ -319,6 +321,46 @@ def silu_mul(gate_up):
     with torch.cuda.device(gate_up.device):
         _check(lib.w4a16_silu_mul(gate_up.data_ptr(), out.data_ptr(), rows, n, _stream(gate_up)), "silu_mul")
     return out
+
+
+def silu_mul_tiles(gate_up):
+    """The same product where 32-wide gate and up tiles alternate along a row, as a fuse_gate_up linear puts them out
+    (see w4a16_silu_mul_tiles in include/w4a16_b200.h)."""
+    _check_tensor(gate_up, "gate_up", dtype=torch.float16)
+    n = gate_up.shape[-1] // 2
+    rows = gate_up.numel() // (2 * n)
+    out = torch.empty(tuple(gate_up.shape[:-1]) + (n,), dtype=torch.float16, device=gate_up.device)
+    lib = load_library()
+    with torch.cuda.device(gate_up.device):
+        _check(lib.w4a16_silu_mul_tiles(gate_up.data_ptr(), out.data_ptr(), rows, n, _stream(gate_up)), "silu_mul_tiles")
+    return out
+
+
+def append_qkv(qkv, k_cache, v_cache, pos0: int, heads: int, rope=None):
+    """Rotary embedding on q (in place in `qkv`) and k, and keys and values of a prompt appended to the static cache
+    (see w4a16_append_qkv in include/w4a16_b200.h).  qkv fp16 [B, S, >= 3*heads*D] contiguous, k_cache / v_cache fp16
+    [B, heads, max_len, D] (updated in place at rows pos0 .. pos0+S-1), rope = (cos, sin) fp16 [>= S, D] tables that start
+    at position pos0, or None."""
+    _check_tensor(qkv, "qkv", dtype=torch.float16, dims=3)
+    _check_tensor(k_cache, "k_cache", dtype=torch.float16, dims=4)
+    _check_tensor(v_cache, "v_cache", dtype=torch.float16, dims=4)
+    B, H, max_len, D = k_cache.shape
+    S = qkv.shape[1]
+    _need(H == int(heads) and tuple(v_cache.shape) == tuple(k_cache.shape), "cache shape must be [B, heads, max_len, D]")
+    _need(qkv.shape[0] == B and qkv.shape[2] >= 3 * H * D, "qkv must be [B, S, >= 3*heads*D]")
+    _need(0 <= int(pos0) and int(pos0) + S <= max_len, "positions must lie inside the cache")
+    cos = sin = None
+    if rope is not None:
+        cos, sin = rope
+        _check_tensor(cos, "rope cos", dtype=torch.float16, dims=2)
+        _check_tensor(sin, "rope sin", dtype=torch.float16, dims=2)
+        _need(cos.shape[1] == D and sin.shape == cos.shape and cos.shape[0] >= S, "rope tables must be [>= S, D]")
+    lib = load_library()
+    with torch.cuda.device(qkv.device):
+        st = lib.w4a16_append_qkv(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), cos.data_ptr() if cos is not None else None,
+                                  sin.data_ptr() if sin is not None else None, B, S, H, D, max_len, int(pos0), qkv.shape[2],
+                                  _stream(qkv))
+    _check(st, "append_qkv")
 
 
 def decode_attention(qkv, k_cache, v_cache, pos, heads: int, rope=None, scale=None, out=None):

@@ -147,6 +147,8 @@ class DecoderLayer(nn.Module):
 
     def forward(self, x, pos0: int, rope=None):
         B, S, H = x.shape
+        if x.is_cuda and H <= 8192 and H % 8 == 0 and self.head_dim % 16 == 0:
+            return self._forward_kernels(x, pos0, rope)
         h = self.ln1(x)
         q, k, v = self.qkv_proj(h).split(self.local_heads * self.head_dim, dim=-1)
         q = q.view(B, S, self.local_heads, self.head_dim).transpose(1, 2)
@@ -172,6 +174,43 @@ class DecoderLayer(nn.Module):
         return x
 
 
+def _layer_forward_kernels(self, x, pos0: int, rope=None):
+    """DecoderLayer.forward on the GPU: everything between the linears and the attention in the library's own kernels,
+    one pass over memory each (an OPT-shaped layer of 8 x 512 tokens spent 250 us in torch's elementwise and copy kernels,
+    a LLaMA-shaped one of 3 x 333 tokens 350 us, as much as in its linears; a prefill of four layers 6580 -> 5980 us and
+    3138 -> 1886 us with them gone)."""
+    from quant import add_norm, append_qkv, silu_mul_tiles
+    B, S, H = x.shape
+    D, heads = self.head_dim, self.local_heads
+    # from 256 tokens on the residual and the ReLU go into the linears' epilogues, where they hide behind the next
+    # tile's MMAs; below, the linears run a wave or less and an epilogue that waits for more data is on the critical path
+    fold = B * S >= 256
+    x = x if x.is_contiguous() else x.contiguous()
+    _, h = add_norm(x, None, *_norm_args(self.ln1))
+    qkv = self.qkv_proj(h)
+    append_qkv(qkv, self.k_cache, self.v_cache, pos0, heads, rope)
+    q = qkv[..., :heads * D].view(B, S, heads, D).transpose(1, 2)
+    keys, vals = self.k_cache[:, :, :pos0 + S], self.v_cache[:, :, :pos0 + S]
+    a = F.scaled_dot_product_attention(q, keys, vals, is_causal=(S > 1 and pos0 == 0))
+    a = a.transpose(1, 2).reshape(B, S, heads * D)
+    if fold:
+        x = self.out_proj(a, residual=x)
+        _, h = add_norm(x, None, *_norm_args(self.ln2))
+    else:
+        x, h = add_norm(x, self.out_proj(a), *_norm_args(self.ln2))
+    if self.cfg.kind == "opt":
+        h = h.reshape(1, B * S, H)
+        f = self.fc1(h, relu=True) if fold else torch.relu(self.fc1(h))
+    else:
+        f = silu_mul_tiles(self.gate_up_proj(h))
+    if fold:
+        return self.fc2(f, residual=x.view(f.shape[:-1] + (H,))).view(B, S, H)
+    return x + self.fc2(f).reshape(B, S, H)
+
+
+DecoderLayer._forward_kernels = _layer_forward_kernels
+
+
 def _norm_args(norm):
     """(weight, bias, eps, rms) of an nn.LayerNorm or RMSNorm, as quant.add_norm takes them."""
     if isinstance(norm, RMSNorm):
@@ -188,7 +227,7 @@ def _layer_forward_static(self, x, pos_t, rope, stats=None):
     buffer for the attention block's output, buffer for this layer's output).  The fused q/k/v GEMV feeds the decode
     attention kernel, which also appends to the cache and applies the rotary embedding (`rope` = the full (cos, sin)
     tables or None).  Returns the new residual stream."""
-    from quant import add_norm, decode_attention, silu_mul
+    from quant import add_norm, decode_attention, silu_mul_tiles
     B, S, H = x.shape
     if stats is None:
         _, h = add_norm(x, None, *_norm_args(self.ln1))
@@ -199,8 +238,7 @@ def _layer_forward_static(self, x, pos_t, rope, stats=None):
             return x + self.fc2(self.fc1(h.reshape(1, B, H), relu=True)).reshape(B, 1, H)
         if B <= 32:
             return x + self.fc2(self.gate_up_proj(h, silu_mul=True))
-        gate, up = split_gate_up(self.gate_up_proj(h))
-        return x + self.fc2(silu_mul(torch.cat((gate, up), dim=-1)))
+        return x + self.fc2(silu_mul_tiles(self.gate_up_proj(h)))
     s_in, s_mid, s_out = stats
     qkv = self.qkv_proj(x, pre_norm=(*_norm_args(self.ln1), s_in)).view(B, -1)
     a = decode_attention(qkv, self.k_cache, self.v_cache, pos_t, self.local_heads, rope=rope).view(B, 1, -1)
@@ -279,7 +317,12 @@ class Decoder(nn.Module):
         for layer in self.layers:
             x = layer(x, self.pos, rope)
         self.pos += S
-        h = self.final_norm(x[:, -1])
+        h = x[:, -1]
+        if h.is_cuda and h.shape[-1] <= 8192 and h.shape[-1] % 8 == 0:
+            from quant import add_norm
+            h = add_norm(h.contiguous(), None, *_norm_args(self.final_norm))[1]
+        else:
+            h = self.final_norm(h)
         logits = h @ self.lm_head.t()
         if self.world > 1:
             sizes = [b - a for a, b in self.vocab_ranges]

@@ -137,3 +137,45 @@ def test_decode_attention_context_split_over_a_cluster():
             _case(B=2, H=3, D=64, L=320, pos=319, rope=True, seed=split)
     finally:
         lib.w4a16_tune_attention(0)
+
+
+@pytest.mark.parametrize("rope", [False, True])
+@pytest.mark.parametrize("B,S,H,D,L,pos0,pad", [(1, 1, 1, 16, 4, 3, 0), (3, 7, 5, 64, 16, 0, 8), (2, 33, 4, 128, 40, 5, 0), (1, 300, 2, 128, 300, 0, 64)])
+def test_append_qkv_against_the_torch_ops(rope, B, S, H, D, L, pos0, pad):
+    """Keys and values land in rows pos0 .. pos0+S-1 of the cache and nowhere else, exactly without rotation; with it q
+    (in place) and k are one rounding away from the float64 rotation (relative 2^-11 of the larger product)."""
+    import quant
+    g = torch.Generator().manual_seed(S + D)
+    qkv = torch.randn(B, S, 3 * H * D + pad, generator=g).half()
+    kc, vc = torch.randn(B, H, L, D, generator=g).half(), torch.randn(B, H, L, D, generator=g).half()
+    ang = torch.rand(S, D // 2, generator=g) * 6.28
+    emb = torch.cat((ang, ang), dim=-1)
+    cos, sin = emb.cos().half(), emb.sin().half()
+    dq, dk, dv = qkv.cuda(), kc.cuda(), vc.cuda()
+    quant.append_qkv(dq, dk, dv, pos0, H, (cos.cuda(), sin.cuda()) if rope else None)
+    q, k, v = (qkv[..., i * H * D:(i + 1) * H * D].reshape(B, S, H, D).transpose(1, 2).double() for i in range(3))
+
+    def rot(t):
+        return t * cos.double() + torch.cat((-t[..., D // 2:], t[..., :D // 2]), -1) * sin.double() if rope else t
+
+    tol = 2.0 ** -11 * 1.42 if rope else 0.0                      # |x cos - y sin| <= sqrt(2) max(|x|, |y|)
+    big = float(qkv.abs().max())
+    dk, dv, dq = dk.cpu().double(), dv.cpu().double(), dq.cpu()
+    assert (dk[:, :, pos0:pos0 + S] - rot(k)).abs().max() <= tol * big
+    assert (dv[:, :, pos0:pos0 + S] - v).abs().max() == 0
+    assert (dq[..., :H * D].reshape(B, S, H, D).transpose(1, 2).double() - rot(q)).abs().max() <= tol * big
+    assert torch.equal(dq[..., H * D:], qkv[..., H * D:])
+    mask = torch.ones(L, dtype=torch.bool)
+    mask[pos0:pos0 + S] = False
+    assert torch.equal(dk[:, :, mask], kc[:, :, mask].double()) and torch.equal(dv[:, :, mask], vc[:, :, mask].double())
+    with pytest.raises(RuntimeError):
+        quant.append_qkv(qkv.cuda(), kc.cuda(), vc.cuda(), L - S + 1, H)
+
+
+@pytest.mark.parametrize("rows,n", [(1, 32), (33, 96), (999, 1376)])
+def test_silu_mul_of_alternating_tiles(rows, n):
+    import quant
+    from w4a16.tp import split_gate_up
+    y = (torch.randn(1, rows, 2 * n, generator=torch.Generator().manual_seed(n)) * 3).half().cuda()
+    gate, up = split_gate_up(y)
+    assert torch.equal(quant.silu_mul_tiles(y), quant.silu_mul(torch.cat((gate, up), dim=-1).contiguous()))

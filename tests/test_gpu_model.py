@@ -80,3 +80,44 @@ def test_token_step_with_folded_normalisations(kind):
         outs.append(nxt)
     assert launches[1] <= launches[0] - 2 * (cfg.layers - 1) - 1     # two launches fewer per layer, one fewer in the first
     assert (outs[0] == outs[1]).float().mean().item() >= 0.66        # greedy tokens of random-weight models: near ties may flip
+
+
+@pytest.mark.parametrize("kind", ["opt", "llama"])
+@pytest.mark.parametrize("B,S", [(3, 40), (2, 150)])                 # epilogues on their own, and inside the linears
+def test_prefill_kernels_match_the_torch_ops(kind, B, S):
+    """DecoderLayer.forward on the library's kernels against the same layers run op by op in torch around the same
+    linears: logits and the filled cache (fp16 rotary arithmetic in torch, one rounding here), then a second chunk behind it."""
+    import torch.nn.functional as F
+    from w4a16.models import Decoder, DecoderConfig, apply_rope
+    from w4a16.tp import split_gate_up
+    cfg = DecoderConfig(kind, layers=2, hidden=512, heads=8, ffn=2048 if kind == "opt" else 1344, vocab=512,
+                        group_size=128 if kind == "opt" else 64, max_positions=256)
+    model = Decoder(cfg, device="cuda", seed=3).mark_static()
+    ids = torch.randint(0, cfg.vocab, (B, S), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+
+    def plain(layer, x, pos0, rope):
+        q, k, v = (t.view(B, -1, 8, 64).transpose(1, 2) for t in layer.qkv_proj(layer.ln1(x)).split(512, dim=-1))
+        n = x.shape[1]
+        if rope is not None:
+            q, k = apply_rope(q, *rope), apply_rope(k, *rope)
+        layer.k_cache[:, :, pos0:pos0 + n], layer.v_cache[:, :, pos0:pos0 + n] = k, v
+        a = F.scaled_dot_product_attention(q, layer.k_cache[:, :, :pos0 + n], layer.v_cache[:, :, :pos0 + n], is_causal=n > 1 and pos0 == 0)
+        x = x + layer.out_proj(a.transpose(1, 2).reshape(B, n, 512))
+        h = layer.ln2(x)
+        if kind == "opt":
+            return x + layer.fc2(torch.relu(layer.fc1(h)))
+        gate, up = split_gate_up(layer.gate_up_proj(h))
+        return x + layer.fc2(F.silu(gate) * up)
+
+    got = []
+    for fused in (True, False):
+        model.reset(B, S + 1)
+        if not fused:
+            for layer in model.layers:
+                layer.forward = lambda x, pos0, rope, layer=layer: plain(layer, x, pos0, rope)
+        logits = model(ids)
+        nxt = model(ids[:, :1])
+        got.append([logits, nxt] + [t for la in model.layers for t in (la.k_cache, la.v_cache)])
+    for a, b in zip(*got):
+        rel = ((a.float() - b.float()).norm() / b.float().norm()).item()
+        assert rel <= 1e-2, rel                                    # fp16 stacks: one rounding in a layer travels through the rest
