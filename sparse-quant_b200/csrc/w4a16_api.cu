@@ -77,20 +77,29 @@ EncodeTiledFn get_encode_fn()
 }
 }  // namespace
 
-int encode_tensor_map_2d(void* tmap, const void* base, int elem_bytes, const uint64_t dims[2], uint64_t row_stride_bytes,
-                         const uint32_t box[2], bool swizzle128)
+int encode_tensor_map(void* tmap, const void* base, int elem_bytes, int rank, const uint64_t* dims, const uint64_t* strides,
+                      const uint32_t* box, bool swizzle128)
 {
     EncodeTiledFn encode = get_encode_fn();
     if (!encode) return record_cuda_error(cudaErrorNotSupported);
-    const cuuint64_t gdims[2] = {dims[0], dims[1]};
-    const cuuint64_t gstr[1] = {row_stride_bytes};
-    const cuuint32_t gbox[2] = {box[0], box[1]};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUtensorMapDataType dt = elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT32;
-    CUresult r = encode((CUtensorMap*)tmap, dt, 2, const_cast<void*>(base), gdims, gstr, gbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    cuuint64_t gdims[3], gstr[2];
+    cuuint32_t gbox[3];
+    const cuuint32_t estr[3] = {1, 1, 1};
+    for (int i = 0; i < rank; ++i) { gdims[i] = dims[i]; gbox[i] = box[i]; }
+    for (int i = 0; i + 1 < rank; ++i) gstr[i] = strides[i];
+    const CUtensorMapDataType dt = elem_bytes == 2   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                   : elem_bytes == 8 ? CU_TENSOR_MAP_DATA_TYPE_UINT64
+                                                     : CU_TENSOR_MAP_DATA_TYPE_UINT32;
+    CUresult r = encode((CUtensorMap*)tmap, dt, (cuuint32_t)rank, const_cast<void*>(base), gdims, gstr, gbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? W4A16_OK : record_cuda_error(cudaErrorInvalidValue);
+}
+
+int encode_tensor_map_2d(void* tmap, const void* base, int elem_bytes, const uint64_t dims[2], uint64_t row_stride_bytes,
+                         const uint32_t box[2], bool swizzle128)
+{
+    return encode_tensor_map(tmap, base, elem_bytes, 2, dims, &row_stride_bytes, box, swizzle128);
 }
 
 void skinny_force_config(int wn, int splits);
@@ -98,6 +107,7 @@ void skinny_set_timeline(unsigned long long* buf);
 void gemv_force_config(int tn, int splits, int depth);
 void gemv_set_timeline(unsigned long long* buf);
 void decode_force_kernel(int which);
+void narrow_force_config(int blocks, int splits);
 int gemv_plan(int tokens, int N, int K, int g, int* plan);
 void gemv_force_ahead(int units);
 void tc_force_config(int tile_tokens, int split_k);
@@ -186,11 +196,18 @@ extern "C" int w4a16_gemm_fused(const void* x, const void* qweight, const void* 
     a.relu = (flags & W4A16_FLAG_RELU) != 0;
     a.silu_mul = (flags & W4A16_FLAG_SILU_MUL) != 0;
 
+    const int forced = decode_forced_kernel();
+    const bool narrow = forced == 3 ? algo != W4A16_ALGO_TC && narrow_supported(tokens, N, K, group_size)
+                                    : forced == 0 && algo == W4A16_ALGO_AUTO && narrow_preferred(tokens, N, K, group_size);
     if (algo == W4A16_ALGO_AUTO) algo = (tokens <= 32 || !tc_supported(tokens, N, K, group_size)) ? W4A16_ALGO_SKINNY : W4A16_ALGO_TC;
     if (a.silu_mul) {
         // the SwiGLU epilogue lives in the decode kernels (one pass of at most 32 tokens); larger inputs use
         // w4a16_silu_mul on the plain output
         if (algo != W4A16_ALGO_SKINNY || tokens > 32 || (N % 64) || residual) return W4A16_ERR_BAD_ALGO;
+    }
+    if (narrow) {
+        s = launch_narrow(a, (cudaStream_t)stream);
+        if (s != W4A16_ERR_BAD_ALGO || forced == 3) return s;         // no launch shape: the kernels below
     }
     if (algo == W4A16_ALGO_TC) {
         if (!tc_supported(tokens, N, K, group_size)) return W4A16_ERR_BAD_ALGO;
@@ -339,7 +356,8 @@ extern "C" void w4a16_tune_skinny(int wn, int splits) { skinny_force_config(wn, 
 extern "C" void w4a16_tune_decode(int kernel, int tiles_per_cta, int splits, int depth)
 {
     decode_force_kernel(kernel);
-    gemv_force_config(tiles_per_cta, splits, depth);
+    gemv_force_config(kernel == 3 ? 0 : tiles_per_cta, kernel == 3 ? 0 : splits, kernel == 3 ? 0 : depth);
+    narrow_force_config(kernel == 3 ? tiles_per_cta : 0, kernel == 3 ? splits : 0);
 }
 extern "C" void w4a16_tune_decode_prefetch(int units_ahead) { gemv_force_ahead(units_ahead); }
 extern "C" int w4a16_debug_decode_plan(int tokens, int N, int K, int group_size, int* plan9)

@@ -202,13 +202,22 @@ cudaError_t launch_after_previous(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
 int  record_cuda_error(cudaError_t e);          // returns W4A16_ERR_CUDA, remembers e
 void count_launch(unsigned n = 1);
 int* device_error_word();
-// cuTensorMapEncodeTiled for a row-major 2-D tensor (dims = {inner, outer} in elements); `tmap` is a CUtensorMap*
+// cuTensorMapEncodeTiled for a tensor of `rank` dimensions, innermost first (strides in bytes, without the innermost
+// one's); `tmap` is a CUtensorMap*
+int encode_tensor_map(void* tmap, const void* base, int elem_bytes, int rank, const uint64_t* dims, const uint64_t* strides,
+                      const uint32_t* box, bool swizzle128);
+// the same for a row-major 2-D tensor (dims = {inner, outer} in elements)
 int encode_tensor_map_2d(void* tmap, const void* base, int elem_bytes, const uint64_t dims[2], uint64_t row_stride_bytes,
                          const uint32_t box[2], bool swizzle128);                       // per-device word a kernel sets to 1 when a bounded wait gives up
 
 // decode path: tokens <= 16 per pass -> launch_gemv (8-warp CTAs, two per SM), otherwise the 16-warp kernel
 int launch_skinny(const GemmArgs& a, cudaStream_t st);
 int launch_gemv(const GemmArgs& a, cudaStream_t st);
+// batched decode on the tensor cores (w4a16_narrow.cu); W4A16_ERR_BAD_ALGO: no launch shape fits
+int launch_narrow(const GemmArgs& a, cudaStream_t st);
+bool narrow_supported(int tokens, int N, int K, int g);
+bool narrow_preferred(int tokens, int N, int K, int g);
+int decode_forced_kernel();                       // 0: none (w4a16_tune_decode)
 // how long a kernel waits for a peer's partial sums in the exchange buffers before it gives up (w4a16_tune_exchange_wait)
 unsigned long long exchange_wait_budget_ns();
 // err_word: device word raised on a barrier timeout (nullptr = the library's per-device word)

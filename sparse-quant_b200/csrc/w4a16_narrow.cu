@@ -1,0 +1,610 @@
+// Batched-decode kernel: W4A16 GEMM for a few dozen tokens on the 5th-generation tensor cores.
+//
+//   out[t, n] = fp16( sum_g s[n, g] * sum_{k in g} (q[n, k] - z[n, g]) * x[t, k] ) (+ bias[n])
+//
+// Replaces the 16-wide and 32-wide instantiations of gemm_s4_f16_nn (gemm_template.h:358-464, gemm_s4_f16.cu:66-87 of the
+// reference).  Bound: the packed weights' way from HBM.  With mma.sync the batch is paid for in issue slots (8.2 cycles
+// per m16n8k16 and scheduler, four of them per 16 x 16 weights at 32 tokens); here the cost of a weight does not depend
+// on the batch: it is unpacked once, written to tensor memory and multiplied by tcgen05.mma.
+//
+// The arithmetic keeps the decode kernels' precision: what goes into the MMA is the integer q - z (exact in fp16), a
+// quantisation group accumulates in fp32 in tensor memory, and the scale is applied in fp32 when the group's sums are
+// added up in registers - the weight is never rounded to fp16 (a denormal scale is flushed, as mul.ftz does).
+//
+// One CTA per SM, warp specialised; a unit of work (stage) is 128 out-features x 128 k:
+//   warps 0, 3  weights: one tensor copy of the four k-tile rows of four packed tiles, one of the (zero, scale) rows; a ring
+//               as deep as shared memory allows (about 100 KB in flight); under programmatic launch they start before the
+//               previous grid has ended
+//   warp 1      activations: one tensor copy of two swizzled 64-k sub-tiles of T tokens.  One copy a stage and producer: with
+//               two in one warp the producers' loops took 700 cycles a stage and set the pace
+//   warp 2      tcgen05.mma, eight per stage, one commit
+//   warps 4-19  dequantisers: a warp takes a 32-feature quarter of a stage, four sets of four take stages in turn (a barrier
+//               round trip costs as much as unpacking a tile: a task of four tiles, not two)
+//   warps 20..  scale and accumulate: tcgen05.ld of a group's sums, acc += s * sum, 16 tokens a warp (32 of the 64-token tile)
+// Two barriers per stage tie the three together: `ready` (dequantised weights written, activations arrived, group sums
+// of the slot's last user read: one probe for the MMA warp, whose loop sets the pace - with a barrier for each it issued a
+// stage every 600 cycles, and eight MMAs take 360) and `done` (the stage's MMAs have completed).  Ring indexes run on
+// across the CTA's out-feature blocks.  Edges need no code: copies past N, K or the tokens arrive as zeros, and a missing
+// group's scale is zero.
+//
+// Split of the work: a cluster of S CTAs takes b out-feature blocks and splits K; the partial sums meet in shared memory
+// and are added over the cluster in rank order (deterministic, no scratch in global memory, capturable).  Every mbarrier
+// wait is bounded; a timeout raises the device error word.
+#include <cooperative_groups.h>
+#include <cuda.h>
+
+#include "w4a16_common.cuh"
+#include "w4a16_sm100.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace w4a16 {
+
+using namespace sm100;
+
+namespace {
+
+constexpr int kBlockN = 128, kBlockK = 128;
+constexpr uint64_t kWaitBudgetNs = 400ull * 1000 * 1000;
+constexpr int kMaxStages = 16;
+constexpr int kFirstDequantWarp = 4, kFirstEpilogueWarp = 20;
+constexpr int kNarrowSmem = 227 * 1024;
+
+template <int T, int G>
+struct NarrowCfg {
+    static constexpr int kGroups = kBlockK / G;                          // quantisation groups per stage
+    static constexpr int kRing = T == 64 ? 4 : 6;                        // A ring, in stages
+    static constexpr int kDRing = T == 32 && G == 64 ? 2 : (T == 64 && G == 64 ? 2 : 4);     // group sums, in stages
+    static constexpr int kDCol = 64 * kRing;                             // first tensor memory column of the sums
+    static constexpr int kXSub = T * 128, kXStage = 2 * kXSub;           // bytes
+    static constexpr int kWStage = 16 * 512 + kGroups * 512;
+    static constexpr int kEpiCols = T < 64 ? 16 : 32;                    // tokens per epilogue warp
+    static constexpr int kEpiWarps = 4 * (T / kEpiCols);
+    static constexpr int kThreads = 32 * (kFirstEpilogueWarp + kEpiWarps);
+    static constexpr int kBarriers = 4 * kMaxStages;
+    static constexpr int kBarBytes = 1024;
+    static constexpr int kRedBytes = T * kBlockN * 4;                    // fp32 sums of one out-feature block
+    static_assert(kDCol + T * kGroups * kDRing <= 512, "tensor memory");
+    static_assert(8 * kBarriers + 8 <= kBarBytes, "barrier area");
+    static int stages(int blocks)                                        // depth of the weight and activation rings
+    {
+        const int room = (kNarrowSmem - 1024 - kBarBytes - blocks * kRedBytes) / (kXStage + kWStage);
+        return room < kMaxStages ? room : kMaxStages;
+    }
+};
+
+struct NarrowParams {
+    const uint32_t* zs;
+    const __half*   bias;
+    const __half*   residual;
+    __half*         out;
+    int*            error;
+    int tokens, N, K;
+    int n_blocks;        // out-feature blocks of the matrix
+    int blocks;          // out-feature blocks per cluster
+    int splits;          // CTAs per cluster: parts of K
+    int stages;          // Q: depth of the rings in shared memory and of the barriers
+    int relu, silu_mul, pdl;
+};
+
+__device__ __forceinline__ float ld_cluster_f32(uint32_t local_addr, uint32_t rank)
+{
+    uint32_t remote;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+    return v;
+}
+
+// (64 + q) - (64 + z) of two lanes: exact, both are fp16 numbers of the same few binades
+__device__ __forceinline__ uint32_t sub_h2(uint32_t a, uint32_t b)
+{
+    uint32_t r;
+    asm("sub.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+
+template <int T, int G>
+__global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map,
+                                                                           const __grid_constant__ CUtensorMap zs_map, const NarrowParams p)
+{
+    using Cfg = NarrowCfg<T, G>;
+    constexpr int R = Cfg::kRing, DR = Cfg::kDRing, GPS = Cfg::kGroups;
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    unsigned char* smem = smem_raw + (smem_base - smem_u32(smem_raw));
+    const int Q = p.stages;
+    const uint32_t w_off = Q * Cfg::kXStage, red_off = w_off + Q * Cfg::kWStage, bar_off = red_off + p.blocks * Cfg::kRedBytes;
+    const uint32_t bar_base = smem_base + bar_off;
+    auto ready_bar  = [&](int s) { return bar_base + 8u * s; };
+    auto done_bar   = [&](int s) { return bar_base + 8u * (kMaxStages + s); };
+    auto wfull_bar  = [&](int s) { return bar_base + 8u * (2 * kMaxStages + s); };
+    auto wempty_bar = [&](int s) { return bar_base + 8u * (3 * kMaxStages + s); };
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + bar_off + 8 * Cfg::kBarriers);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const uint32_t red_base = smem_base + red_off;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (p.pdl) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int k_steps = (p.K + kBlockK - 1) / kBlockK;
+    const int S = p.splits, rank = blockIdx.y;
+    const int ks0 = k_steps * rank / S, ks1 = k_steps * (rank + 1) / S;
+    const int nb0 = blockIdx.x * p.blocks, nblk = min(p.blocks, p.n_blocks - nb0);
+    const int total = nblk * (ks1 - ks0);                            // stages of this CTA
+    auto load_weights = [&](int sw, int nb, int ks) {                // one elected lane
+        const uint32_t dst = smem_base + w_off + sw * Cfg::kWStage, bar = wfull_bar(sw);
+        mbar_arrive_expect_tx(bar, 8192);
+        tma_load_2d(dst, &w_map, nb * 256, ks * 4, bar);
+    };
+    constexpr int kEarly = 2;                                        // stages requested before the rest of the CTA is set up
+    if (warp == 0) {
+        if (lane < Q) {
+            mbar_init(ready_bar(lane), 4 + Cfg::kEpiWarps + 1); mbar_init(done_bar(lane), 1);
+            mbar_init(wfull_bar(lane), 2); mbar_init(wempty_bar(lane), 4);
+        }
+        mbar_fence_init();
+        __syncwarp();
+    }
+    if (threadIdx.x == 0) {
+        *abort_flag = 0;
+        for (int i = 0; i < kEarly && i < ks1 - ks0; ++i) load_weights(i, nb0, ks0 + i);
+    }
+    if (warp == 3) {
+        tmem_alloc(smem_u32((const void*)tmem_slot), 512);
+        tmem_relinquish();
+    }
+    if (warp == 1 && lane == 0) prefetch_tmap(&x_map);
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        // ---- packed weights ----
+        int st = 0, nb = nb0, ks = ks0; uint32_t phase = 0;
+        bool ok = true;
+        for (int it = 0; it < total; ++it) {
+            if (it >= Q && !(ok = __all_sync(0xffffffffu, mbar_wait(wempty_bar(st), phase ^ 1u, abort_flag, kWaitBudgetNs)))) break;
+            if ((it >= kEarly || it >= ks1 - ks0) && elect_one()) load_weights(st, nb, ks);
+            __syncwarp();
+            if (++ks == ks1) { ks = ks0; ++nb; }
+            if (++st == Q) { st = 0; phase ^= 1u; }
+        }
+        if (!ok) {                                                   // let copies in flight land before the CTA goes
+            const uint64_t t0 = globaltimer_ns();
+            while (globaltimer_ns() - t0 < 200000) { }
+        }
+    } else if (warp == 1) {
+        // ---- activations ----
+        if (p.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
+        int st = 0, ks = ks0; uint32_t phase = 0;
+        bool ok = true;
+        for (int it = 0; it < total; ++it) {
+            if (it >= Q && !(ok = __all_sync(0xffffffffu, mbar_wait(done_bar(st), phase ^ 1u, abort_flag, kWaitBudgetNs)))) break;
+            if (elect_one()) {
+                mbar_arrive_expect_tx(ready_bar(st), Cfg::kXStage);
+                tma_load_3d(smem_base + st * Cfg::kXStage, &x_map, 0, 0, 2 * ks, ready_bar(st));
+            }
+            __syncwarp();
+            if (++ks == ks1) ks = ks0;
+            if (++st == Q) { st = 0; phase ^= 1u; }
+        }
+        if (!ok) {
+            const uint64_t t0 = globaltimer_ns();
+            while (globaltimer_ns() - t0 < 200000) { }
+        }
+    } else if (warp == 3) {
+        // ---- (zero, scale) rows ----
+        int st = 0, nb = nb0, ks = ks0; uint32_t phase = 0;
+        bool ok = true;
+        for (int it = 0; it < total; ++it) {
+            if (it >= Q && !(ok = __all_sync(0xffffffffu, mbar_wait(wempty_bar(st), phase ^ 1u, abort_flag, kWaitBudgetNs)))) break;
+            if (elect_one()) {
+                mbar_arrive_expect_tx(wfull_bar(st), GPS * 512);
+                tma_load_2d(smem_base + w_off + st * Cfg::kWStage + 8192, &zs_map, nb * kBlockN, ks * GPS, wfull_bar(st));
+            }
+            __syncwarp();
+            if (++ks == ks1) { ks = ks0; ++nb; }
+            if (++st == Q) { st = 0; phase ^= 1u; }
+        }
+        if (!ok) {
+            const uint64_t t0 = globaltimer_ns();
+            while (globaltimer_ns() - t0 < 200000) { }
+        }
+    } else if (warp == 2) {
+        // ---- MMA: the whole warp walks the loop, an elected lane issues (see elect_one) ----
+        constexpr uint32_t idesc = idesc_f16_m128(T);
+        const uint64_t bdesc0 = smem_desc_sw128(smem_base);
+        // A probe of a barrier answers after some 200 cycles: each is asked two stages ahead, so that none is waited for.
+        int st = 0, ahead = 0, slot = 0, d = 0; uint32_t phase = 0, ahead_phase = 0;
+        bool ready0 = false, ready1 = false;
+        auto probe = [&]() {
+            const bool r = mbar_test_wait(ready_bar(ahead), ahead_phase);
+            if (++ahead == Q) { ahead = 0; ahead_phase ^= 1u; }
+            return r;
+        };
+        ready0 = probe();
+        ready1 = probe();
+        for (int it = 0; it < total; ++it) {
+            if (!ready0 && !mbar_wait(ready_bar(st), phase, abort_flag, kWaitBudgetNs)) break;     // the same for every lane
+            __syncwarp();
+            tc_fence_after_sync();
+            const bool ready2 = probe();
+            const uint64_t bdesc = bdesc0 + (uint64_t)((uint32_t)(st * Cfg::kXStage) >> 4);
+            const uint32_t a_tmem = tmem_base + 64 * slot, d_tmem = tmem_base + Cfg::kDCol + d * (GPS * T);
+            if (elect_one()) {
+#pragma unroll
+                for (int kk = 0; kk < 8; ++kk)
+                    mma_f16_ts(d_tmem + (GPS == 2 && kk >= 4 ? T : 0), a_tmem + 8 * kk,
+                               bdesc + (uint64_t)((kk >= 4 ? (Cfg::kXSub >> 4) : 0) + 2 * (kk & 3)), idesc, (GPS == 2 ? kk & 3 : kk) != 0);
+                tc_commit(done_bar(st));
+            }
+            __syncwarp();
+            if (++st == Q) { st = 0; phase ^= 1u; }
+            if (++slot == R) slot = 0;
+            if (++d == DR) d = 0;
+            ready0 = ready1;
+            ready1 = ready2;
+        }
+    } else if (warp >= kFirstDequantWarp && warp < kFirstEpilogueWarp) {
+        // ---- dequantisers: tensor memory lane quarter = packed tile column = warp % 4 ----
+        const int quarter = warp & 3, set = (warp - kFirstDequantWarp) >> 2;
+        const uint32_t lane_field = (uint32_t)(quarter * 32) << 16;
+        auto step = [](int& i, int by, int n) { i += by; const bool wrap = i >= n; if (wrap) i -= n; return wrap; };
+        int st = set, slot = set % R, freed = set + Q - R; uint32_t phase = 0, freed_phase = 1;    // freed: the stage R back, whose A slot is taken
+        if (freed >= Q) { freed -= Q; freed_phase = 0; }
+        for (int it = set; it < total; it += 4) {
+            {
+                const bool loaded = mbar_test_wait(wfull_bar(st), phase);            // both probes in flight together
+                const bool slot_free = it < R || mbar_test_wait(done_bar(freed), freed_phase);
+                if (!loaded && !mbar_wait(wfull_bar(st), phase, abort_flag, kWaitBudgetNs)) break;    // the same for every lane
+                __syncwarp();
+                const unsigned char* wst = smem + w_off + st * Cfg::kWStage;
+                const uint4* wq = reinterpret_cast<const uint4*>(wst) + quarter * 32 + lane;
+                const uint32_t* zsp = reinterpret_cast<const uint32_t*>(wst + 8192) + quarter * 32 + (lane >> 2);
+                uint4 q[4];
+                uint32_t zz[GPS][4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) q[i] = wq[128 * i];
+#pragma unroll
+                for (int gi = 0; gi < GPS; ++gi)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const uint32_t z = zsp[128 * gi + 8 * i];
+                        zz[gi][i] = __byte_perm(z, z, 0x1010);
+                    }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(wempty_bar(st));
+                if (!slot_free && !mbar_wait(done_bar(freed), freed_phase, abort_flag, kWaitBudgetNs)) break;
+                __syncwarp();
+                tc_fence_after_sync();
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int gi = GPS == 2 ? half : 0;
+                    const uint32_t words[2][4] = {{q[2 * half].x, q[2 * half].y, q[2 * half].z, q[2 * half].w},
+                                                  {q[2 * half + 1].x, q[2 * half + 1].y, q[2 * half + 1].z, q[2 * half + 1].w}};
+#pragma unroll
+                    for (int nh = 0; nh < 2; ++nh) {
+                        uint32_t a[16];
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+#pragma unroll
+                            for (int kh = 0; kh < 2; ++kh) {
+                                uint32_t h[4];
+                                unpack_s4x8(words[i][kh * 2 + nh], h);
+                                uint32_t* o = a + i * 8 + kh * 4;
+                                o[0] = sub_h2(h[0], zz[gi][nh * 2]);
+                                o[1] = sub_h2(h[1], zz[gi][nh * 2 + 1]);
+                                o[2] = sub_h2(h[2], zz[gi][nh * 2]);
+                                o[3] = sub_h2(h[3], zz[gi][nh * 2 + 1]);
+                            }
+                        tmem_st_16x128b_x8(tmem_base + lane_field + ((uint32_t)(nh * 16) << 16) + 64 * slot + 32 * half, a);
+                    }
+                }
+                tmem_wait_st();
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(ready_bar(st));
+            }
+            if (step(st, 4, Q)) phase ^= 1u;
+            step(slot, 4 % R, R);
+            if (step(freed, 4, Q)) freed_phase ^= 1u;
+        }
+    } else if (warp >= kFirstEpilogueWarp) {
+        // ---- scale and accumulate: thread = out-feature (tensor memory lane), registers = tokens ----
+        constexpr int EC = Cfg::kEpiCols;
+        const int quarter = warp & 3, col0 = ((warp - kFirstEpilogueWarp) >> 2) * EC;
+        const uint32_t lane_field = (uint32_t)(quarter * 32) << 16;
+        bool ok = true;
+        if (lane == 0)
+            for (int i = 0; i < DR && i < total; ++i) mbar_arrive(ready_bar(i));          // the first sums find their slots free
+        // The scales come straight from global memory, four stages ahead of their use (the dequantisers' copy has just
+        // brought the line into L2): no barrier, and the weight ring is not held up.
+        constexpr int kAhead = 4;
+        const int groups = p.K / G;
+        uint32_t zs[kAhead][GPS];
+        int fnb = nb0, fks = ks0;                                 // the stage of the next fetch
+        auto fetch = [&](uint32_t (&w)[GPS]) {
+            const int n = min(fnb * kBlockN + quarter * 32 + lane, p.N - 1);
+#pragma unroll
+            for (int gi = 0; gi < GPS; ++gi) {
+                const int g = fks * GPS + gi;
+                w[gi] = g < groups ? ldg_nc_u32(p.zs + (size_t)g * p.N + n) : 0u;
+            }
+            if (++fks == ks1) { fks = ks0; ++fnb; }
+        };
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) if (i < total) fetch(zs[i]);
+        int st = 0, d = 0, free_st = DR % Q, left = ks1 - ks0; uint32_t phase = 0;     // free_st: the stage that gets this sum's slot next
+        float acc[EC];
+#pragma unroll
+        for (int i = 0; i < EC; ++i) acc[i] = 0.f;
+        float* red = reinterpret_cast<float*>(smem + red_off) + col0 * kBlockN + quarter * 32 + lane;
+        for (int base = 0; base < total && ok; base += kAhead) {
+            // unrolled over the scales in flight: handing them down a register queue would wait for the newest load
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const int it = base + u;
+                if (it >= total) break;
+                ok = __all_sync(0xffffffffu, mbar_wait(done_bar(st), phase, abort_flag, kWaitBudgetNs));
+                if (!ok) break;
+                tc_fence_after_sync();
+                float s0[GPS];
+#pragma unroll
+                for (int gi = 0; gi < GPS; ++gi) {
+                    uint32_t v = zs[u][gi];
+                    asm("mul.ftz.f16x2 %0, %1, %2;" : "=r"(v) : "r"(v), "r"(0x3c003c00u));   // a denormal scale becomes 0, as under mul.ftz
+                    s0[gi] = __half2float(__ushort_as_half((unsigned short)(v >> 16)));
+                }
+                const uint32_t src = tmem_base + lane_field + Cfg::kDCol + d * (GPS * T) + col0;
+#pragma unroll
+                for (int gi = 0; gi < GPS; ++gi)
+#pragma unroll
+                    for (int c = 0; c < EC; c += 16) {
+                        uint32_t v[16];
+                        tmem_ld_32x32b_x16(src + gi * T + c, v);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) acc[c + i] = fmaf(s0[gi], __uint_as_float(v[i]), acc[c + i]);
+                    }
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0 && it + DR < total) mbar_arrive(ready_bar(free_st));
+                if (it + kAhead < total) fetch(zs[u]);
+                if (++free_st == Q) free_st = 0;
+                if (++st == Q) { st = 0; phase ^= 1u; }
+                if (++d == DR) d = 0;
+                if (--left == 0) {                                   // the block is complete
+#pragma unroll
+                    for (int i = 0; i < EC; ++i) { red[i * kBlockN] = acc[i]; acc[i] = 0.f; }
+                    red += Cfg::kRedBytes / 4;
+                    left = ks1 - ks0;
+                }
+            }
+        }
+    }
+
+    // ---- the partial sums of the cluster meet: each rank finishes a slice of the outputs ----
+    __syncwarp();
+    tc_fence_before_sync();
+    __syncthreads();
+    if (*abort_flag && threadIdx.x == 0) atomicExch(p.error, 1);
+    if (warp == 3) {
+        tc_fence_after_sync();
+        tmem_dealloc(tmem_base, 512);
+    }
+    cg::cluster_group cluster = cg::this_cluster();
+    if (S > 1) cluster.sync();
+    if (p.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");    // outputs and residual belong to earlier work until then
+    auto total_of = [&](int blk, int tok, int f) {
+        const uint32_t at = red_base + (uint32_t)(blk * Cfg::kRedBytes + (tok * kBlockN + f) * 4);
+        float v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = q < S ? ld_cluster_f32(at, (uint32_t)q) : 0.f;
+        float s = v[0];
+#pragma unroll
+        for (int q = 1; q < 8; ++q) s += v[q];
+        return s;
+    };
+    auto finish = [&](float s, int n) {
+        __half h = __float2half_rn(s);
+        if (p.bias) h = __hadd(h, p.bias[n]);
+        if (p.relu) h = __hmax(h, __half());
+        return h;
+    };
+    const unsigned rows = (unsigned)p.tokens;
+    if (p.silu_mul) {
+        // gate and up tiles alternate: features f and f + 32 are a pair, one thread owns both (the roundings of the
+        // separate activation and product kernels)
+        const unsigned total = (unsigned)nblk * rows * (kBlockN / 2);
+        const unsigned lo = total * rank / S, hi = total * (rank + 1) / S;
+        for (unsigned e = lo + threadIdx.x; e < hi; e += Cfg::kThreads) {
+            const int pl = e & 63, f = ((pl >> 5) << 6) + (pl & 31);
+            const unsigned bt = e >> 6, blk = bt / rows, tok = bt - blk * rows;
+            const int n = (nb0 + (int)blk) * kBlockN + f;
+            if (n + 32 < p.N) {
+                const float gate = __half2float(finish(total_of(blk, tok, f), n));
+                const __half up = finish(total_of(blk, tok, f + 32), n + 32);
+                p.out[(size_t)tok * (p.N >> 1) + (nb0 + (int)blk) * (kBlockN / 2) + pl] = __hmul(__float2half_rn(gate / (1.f + __expf(-gate))), up);
+            }
+        }
+    } else {
+        const unsigned total = (unsigned)nblk * rows * kBlockN;
+        const unsigned lo = total * rank / S, hi = total * (rank + 1) / S;
+#pragma unroll 2
+        for (unsigned e = lo + threadIdx.x; e < hi; e += Cfg::kThreads) {
+            const int f = e & (kBlockN - 1);
+            const unsigned bt = e >> 7, blk = bt / rows, tok = bt - blk * rows;
+            const int n = (nb0 + (int)blk) * kBlockN + f;
+            if (n < p.N) {
+                __half h = finish(total_of(blk, tok, f), n);
+                const size_t at = (size_t)tok * p.N + n;
+                if (p.residual) h = __hadd(h, p.residual[at]);
+                p.out[at] = h;
+            }
+        }
+    }
+    if (S > 1) cluster.sync();                                       // peers may still be reading this CTA's sums
+}
+
+int g_force_blocks = 0, g_force_splits = 0;
+
+struct NarrowPlan { int blocks, splits, stages; };
+
+template <int T, int G>
+int prepare_instance(int* max_smem_set)
+{
+    static int configured[64] = {0};       // benign race: the attribute call is idempotent
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return record_cuda_error(e);
+    if (dev >= 64 || !configured[dev]) {
+        e = cudaFuncSetAttribute(narrow_kernel<T, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, kNarrowSmem);
+        if (e != cudaSuccess) return record_cuda_error(e);
+        if (dev < 64) configured[dev] = 1;
+    }
+    *max_smem_set = dev;
+    return W4A16_OK;
+}
+
+// clusters of `sp` CTAs the device runs at once (a CTA takes an SM: a property of how the SMs are grouped); cached
+template <int T, int G>
+int max_clusters(int sp)
+{
+    static int cache[64][9] = {};          // benign race: the query is idempotent
+    int dev = 0;
+    if (sp <= 1) return device_sm_count();
+    if (prepare_instance<T, G>(&dev) != W4A16_OK || dev >= 64) return 0;
+    if (cache[dev][sp]) return cache[dev][sp] > 0 ? cache[dev][sp] : 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, sp, 1);
+    cfg.blockDim = dim3(NarrowCfg<T, G>::kThreads);
+    cfg.dynamicSmemBytes = kNarrowSmem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = sp;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, narrow_kernel<T, G>, &cfg) != cudaSuccess) { n = 0; (void)cudaGetLastError(); }
+    cache[dev][sp] = n > 0 ? n : -1;
+    return n;
+}
+
+// Blocks per cluster and cluster size: the fewest stages in the busiest CTA among the shapes that run as one wave; a
+// reduction over a cluster counts as two stages, a shallow weight ring as proportionally slower stages.
+template <int T, int G>
+NarrowPlan plan_narrow(int N, int K)
+{
+    const int n_blocks = (N + kBlockN - 1) / kBlockN, k_steps = (K + kBlockK - 1) / kBlockK;
+    NarrowPlan best = {0, 0, 0};
+    double best_cost = 0;
+    for (int sp = 1; sp <= 8 && sp <= k_steps; ++sp) {
+        if (g_force_splits && sp != g_force_splits) continue;
+        const int room = max_clusters<T, G>(sp);
+        if (room <= 0) continue;
+        int b = (n_blocks + room - 1) / room;
+        if (g_force_blocks) b = g_force_blocks < n_blocks ? g_force_blocks : n_blocks;
+        const int q = NarrowCfg<T, G>::stages(b);
+        if (q < NarrowCfg<T, G>::kRing) continue;
+        const double cost = (double)b * ((k_steps + sp - 1) / sp) * (q >= 10 ? 1.0 : 10.0 / q) + (sp > 1 ? 2.0 : 0.0);
+        if (best.blocks == 0 || cost < best_cost) { best_cost = cost; best = {b, sp, q}; }
+    }
+    return best;
+}
+
+template <int T, int G>
+int launch_instance(const GemmArgs& a, cudaStream_t st)
+{
+    using Cfg = NarrowCfg<T, G>;
+    int dev = 0;
+    int s = prepare_instance<T, G>(&dev);
+    if (s != W4A16_OK) return s;
+    const NarrowPlan pl = plan_narrow<T, G>(a.N, a.K);
+    if (pl.blocks == 0) return W4A16_ERR_BAD_ALGO;
+    CUtensorMap x_map, w_map, zs_map;
+    {
+        // as [K/64][tokens][64]: a box of two is a stage's two swizzled sub-tiles, one copy
+        const uint64_t dims[3] = {64, (uint64_t)a.tokens, (uint64_t)(a.K / 64)}, strides[2] = {(uint64_t)a.K * sizeof(__half), 128};
+        const uint32_t box[3] = {64, (uint32_t)T, 2};
+        s = encode_tensor_map(&x_map, a.x, 2, 3, dims, strides, box, /*swizzle128*/ true);
+        if (s != W4A16_OK) return s;
+    }
+    {
+        // the packed matrix as 64-bit words, one row per k-tile row: a box of four rows of four packed tiles is one copy
+        const uint64_t row_bytes = (uint64_t)(a.N / kTileN) * 512, dims[2] = {row_bytes / 8, (uint64_t)(a.K / kTileK)};
+        const uint32_t box[2] = {256, 4};
+        s = encode_tensor_map_2d(&w_map, a.qw, 8, dims, row_bytes, box, /*swizzle128*/ false);
+        if (s != W4A16_OK) return s;
+    }
+    {
+        const uint64_t dims[2] = {(uint64_t)a.N, (uint64_t)(a.K / G)};
+        const uint32_t box[2] = {(uint32_t)kBlockN, (uint32_t)Cfg::kGroups};
+        s = encode_tensor_map_2d(&zs_map, a.zs, 4, dims, (uint64_t)a.N * 4, box, /*swizzle128*/ false);
+        if (s != W4A16_OK) return s;
+    }
+    NarrowParams p;
+    p.zs = a.zs; p.bias = a.bias; p.residual = a.residual; p.out = a.out;
+    p.error = device_error_word();
+    if (!p.error) return W4A16_ERR_CUDA;
+    p.tokens = a.tokens; p.N = a.N; p.K = a.K;
+    p.n_blocks = (a.N + kBlockN - 1) / kBlockN; p.blocks = pl.blocks; p.splits = pl.splits; p.stages = pl.stages;
+    p.relu = a.relu ? 1 : 0; p.silu_mul = a.silu_mul ? 1 : 0; 
+    p.pdl = a.static_weights && a.tokens <= 32 ? 1 : 0;              // as before: calls of more than 32 tokens keep plain stream order
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((p.n_blocks + pl.blocks - 1) / pl.blocks, pl.splits, 1);
+    cfg.blockDim = dim3(Cfg::kThreads);
+    cfg.dynamicSmemBytes = 1024 + pl.stages * (Cfg::kXStage + Cfg::kWStage) + pl.blocks * Cfg::kRedBytes + Cfg::kBarBytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = pl.splits;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = p.pdl ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, narrow_kernel<T, G>, x_map, w_map, zs_map, p);
+    count_launch();
+    return e == cudaSuccess ? W4A16_OK : record_cuda_error(e);
+}
+
+template <int T>
+int launch_t(const GemmArgs& a, cudaStream_t st)
+{
+    return a.g == 64 ? launch_instance<T, 64>(a, st) : launch_instance<T, 128>(a, st);
+}
+
+}  // namespace
+
+void narrow_force_config(int blocks, int splits) { g_force_blocks = blocks; g_force_splits = splits; }
+
+bool narrow_supported(int tokens, int N, int K, int g)
+{
+    return tokens > 0 && tokens <= 64 && (g == 64 || g == 128) && (K % 64) == 0 && (N % kTileN) == 0;
+}
+
+bool narrow_preferred(int tokens, int N, int K, int g)
+{
+    // Measured in graphs of calls on weights from HBM, us, mma.sync kernels / this one: at 32 tokens 12.8 / 8.5 (4096 -> 4096),
+    // 23.9 / 15.8 (12288), 26.3 / 17.6 (16384), 32.3 / 17.8 (16384 -> 4096), 35.4 / 28.4 (4096 -> 22016, g = 64): from 17 on.
+    // At 9 to 16 tokens they are level with groups of 128 (7.4 / 7.8, 14.9 / 14.1, 15.4 / 15.6, 16.6 / 16.6), this one
+    // ahead with groups of 64, twice the scale work for them (29.6 / 23.3, 15.8 / 13.5).  At 33 to 64 the prefill kernel's
+    // 64-token tile, which does not split K, leaves SMs idle on all but the widest matrices: 20.6 / 9.7 (4096 -> 4096), 28.8 / 20.3
+    // (11008 -> 4096), 21.0 / 21.6 (4096 -> 12288), 41.2 / 42.8 (22016).
+    if (!narrow_supported(tokens, N, K, g)) return false;
+    if (tokens > 32) return N < 12288;
+    return tokens > (g == 64 ? 8 : 16);
+}
+
+int launch_narrow(const GemmArgs& a, cudaStream_t st)
+{
+    if (!narrow_supported(a.tokens, a.N, a.K, a.g)) return W4A16_ERR_BAD_ALGO;
+    if (a.silu_mul && ((a.N % 64) || a.residual)) return W4A16_ERR_BAD_SHAPE;
+    return a.tokens <= 16 ? launch_t<16>(a, st) : a.tokens <= 32 ? launch_t<32>(a, st) : launch_t<64>(a, st);
+}
+
+}  // namespace w4a16

@@ -142,6 +142,9 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const __half* in, __half*
 // de-interleaving into two tensors and torch's two elementwise kernels took about 50.
 __global__ void __launch_bounds__(256) silu_mul_tiles_kernel(const __half* in, __half* out, unsigned n, unsigned total_vec)
 {
+    // as in the kernel above: a GEMV launched with programmatic stream serialization may follow, eagerly or in a graph
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const unsigned nvec = n / 8;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total_vec; i += gridDim.x * blockDim.x) {
         const unsigned r = i / nvec, c = (i - r * nvec) * 8;

@@ -900,8 +900,9 @@ void skinny_force_config(int wn, int splits)
 // debug builds: experiment switches of the kernel (bit 0 no MMAs, bit 1 no activation staging) and a ring-depth cap
 void skinny_debug_mode(int mode, int depth) { g_debug_mode = mode; g_force_depth = depth; }
 
-int g_decode_kernel = 0;      // 0: by measured crossover, 1: always the 16-warp kernel, 2: always the two-CTAs-per-SM kernel
+int g_decode_kernel = 0;      // 0: by measured crossover, 1: always the 16-warp kernel, 2: always the two-CTAs-per-SM kernel, 3: narrow_kernel
 void decode_force_kernel(int which) { g_decode_kernel = which; }
+int decode_forced_kernel() { return g_decode_kernel; }
 
 int launch_skinny(const GemmArgs& a, cudaStream_t st)
 {

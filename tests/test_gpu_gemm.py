@@ -367,3 +367,52 @@ def test_walinear_module_and_host_buffer_entry_point():
                              torch.cuda.current_stream().cuda_stream)
     assert st == 0
     assert torch.equal(oh, y.reshape(M, 128).cpu())
+
+
+@pytest.mark.parametrize("blocks,splits", [(0, 0), (1, 1), (1, 3), (2, 2), (3, 1), (2, 8)])
+def test_narrow_every_decomposition(blocks, splits):
+    """The batched-decode kernel over its launch shapes: out-feature blocks per cluster x cluster size, every token tile
+    (16 / 32 / 64) at its edges, both group sizes, a K that is not a multiple of the 128-k stage, and out-feature counts
+    that leave a block partly and a cluster's last block wholly empty."""
+    import quant
+    lib = quant.load_library()
+    try:
+        lib.w4a16_tune_decode(3, blocks, splits, 0)
+        for (M, N, K, g) in [(1, 96, 1344, 64), (9, 416, 2048, 128), (16, 416, 1344, 64), (17, 96, 1024, 128), (24, 416, 2048, 128),
+                             (32, 1376, 1408, 64), (33, 416, 1344, 64), (64, 416, 2048, 128)]:
+            run(M, N, K, g, algo=0, bias=(M % 2 == 1))
+    finally:
+        lib.w4a16_tune_decode(0, 0, 0, 0)
+    flag = __import__("ctypes").c_int(-1)
+    assert lib.w4a16_device_error_flag(flag) == 0 and flag.value == 0
+
+
+def test_narrow_is_no_less_exact_than_the_decode_kernels_and_keeps_their_epilogues():
+    """The scale is applied in fp32 to exact integer sums: with fp16 rounding of the output only (2^-11 relative to each
+    output, plus fp32 sums) against float64; residual and SwiGLU epilogues round like the launches they replace."""
+    import quant
+    lib = quant.load_library()
+    for (M, n, K, g) in [(9, 704, 1024, 64), (24, 512, 4096, 128), (32, 2752, 4096, 64)]:
+        N = 2 * n
+        p = packed(N, K, g)
+        qw, zs = to_dev(p)
+        x = make_x(M, K)
+        q = lambda **kw: quant.gemm_awq_bias(x.cuda(), qw, zs, None, N, g, **kw)
+        r = torch.randn(1, M, N, generator=torch.Generator().manual_seed(3)).half().cuda()
+        outs = {}
+        try:
+            for kernel in (1, 3):
+                lib.w4a16_tune_decode(kernel, 0, 0, 0)
+                plain, res = q(), q(residual=r)
+                silu = q(silu_mul=True)
+                assert torch.equal(res, plain + r)
+                assert torch.equal(silu, quant.silu_mul_tiles(plain))
+                outs[kernel] = plain[0].double().cpu()
+        finally:
+            lib.w4a16_tune_decode(0, 0, 0, 0)
+        z = torch.from_numpy(p["zs"].view(np.float16).astype(np.float64)).reshape(K // g, N, 2)
+        codes = quant.dequant(qw, torch.stack((torch.full((K // g, N), 64.0), torch.ones(K // g, N)), -1).half().reshape(K // g, 2 * N).cuda(), N, K, g)
+        w = (codes.double().cpu().reshape(N, K // g, g) - (z[..., 0].t()[..., None] - 64.0)) * z[..., 1].t()[..., None]
+        ref = x[0].double() @ w.reshape(N, K).t()
+        err = {k: ((o - ref).norm() / ref.norm()).item() for k, o in outs.items()}
+        assert err[3] <= 1.02 * err[1] and err[3] <= 2.0 ** -11, err       # an fp16 rounding is at most 2^-11 of each output
