@@ -44,7 +44,7 @@ typedef enum w4a16_status {
 
 /* kernel selection for w4a16_gemm_algo */
 typedef enum w4a16_algo {
-    W4A16_ALGO_AUTO   = 0,  /* tokens <= 32: decode kernels; otherwise the tcgen05 kernel */
+    W4A16_ALGO_AUTO   = 0,  /* by tokens and shape: decode kernels (up to 32), batched decode on tcgen05 (9 to 64), prefill */
     W4A16_ALGO_SKINNY = 1,  /* mma.sync decode kernels (up to 8 tokens: two CTAs per SM; up to 32: cluster split-K) */
     W4A16_ALGO_TC     = 2   /* TMA + tcgen05/TMEM GEMM (prefill) */
 } w4a16_algo;
@@ -367,8 +367,9 @@ void w4a16_debug_skinny_timeline(void* buf);
  * 16-warp decode kernel: out-feature tiles per CTA (1,2,4,8,16) and cluster split-K (1..8);
  * tcgen05 kernel: token tile (64,128,256) and K parts per output tile;
  * decode path: kernel (1 = the kernel for up to 32 tokens per pass, 2 = the kernel for up to 8 tokens per pass,
- * 0 = by token count), and for the 8-token kernel out-feature tiles per CTA (1,2,4,8,16), cluster split-K (1..8)
- * and ring depth (2..4). */
+ * 3 = the batched-decode kernel for up to 64 tokens, 0 = by token count), and for the 8-token kernel out-feature tiles
+ * per CTA (1,2,4,8,16), cluster split-K (1..8) and ring depth (2..4), for the batched one 128-wide out-feature blocks
+ * per cluster and cluster size (1..8). */
 void w4a16_tune_skinny(int wn, int splits);
 void w4a16_tune_tc(int tile_tokens, int split_k);
 void w4a16_tune_decode(int kernel, int tiles_per_cta, int splits, int depth);

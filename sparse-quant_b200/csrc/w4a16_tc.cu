@@ -30,12 +30,15 @@
 //            of the stage, written by the dequantisers, read by the MMA.  The commit at the end of a stage releases
 //            the second x sub-tile and the A slot together (barrier `consumed`, waited on by warp 4 and by the
 //            dequantisers).
-//   W ring   (shared memory, own depth): the stage's packed weight tiles (a k-tile row of the format is contiguous:
-//            plain bulk copies) and the (zero, scale) row(s), filled by the last warp, read only by the dequantisers and
+//            The 64- and 128-token tiles move a stage whole: one activation copy, one commit, and a dequantiser's task is
+//            its packed tile column of all 128 k, four sets of four warps taking stages in turn.  A barrier round trip costs
+//            100 to 250 cycles and a copy about 100 to issue, and with two of each per stage and role those tiles took
+//            1000 cycles a stage whatever their size: now 700 (4096 -> 4096: 128 tokens 21.3 -> 16.9 us, 512 24.0 -> 19.7 us;
+//            333 tokens 4096 -> 11008 53 -> 38 us).
+//   W ring   (shared memory, own depth): the stage's packed weight tiles (a box of four k-tile rows by four tiles,
+//            one tensor copy) and the (zero, scale) row(s), filled by the last warp, read only by the dequantisers and
 //            released as soon as they hold the words in registers.
-//   dequantisers (groups of four; a pair of groups takes the two 64-k halves of a stage; with the 64- and
-//            128-token tiles, whose stages are shorter than a pair's latency chain, two pairs take stages in turn -
-//            measured 3-7 % there): read 16 B per lane per 32x32 tile from shared memory, expand the nibbles in
+//   dequantisers (groups of four; with the 256-token tile a pair of groups takes the two 64-k halves of a stage): read 16 B per lane per 32x32 tile from shared memory, expand the nibbles in
 //            registers, (t - z) * s with
 //            sub.ftz/mul.ftz (bit-exact with the reference), and write the fp16 result straight into tensor memory
 //            with tcgen05.st.16x128b - the packed layout is already that fragment order - so the dequantised weights
@@ -66,8 +69,8 @@ constexpr int kBlockK   = 128;                 // k per pipeline stage (4 packed
 constexpr int kSubK     = 64;                  // k per swizzled activation sub-tile (128 bytes of fp16)
 // Warps 4: x TMA; 5: MMA; the last one: W TMA; the other sixteen are workers in groups of four (0-3, 6-9, 10-13, 14-17).
 // Dequantiser groups: with the 256-token tile the first two (one per 64-k half of every stage), the other two being
-// epilogue warps; with the smaller tiles, whose stages are shorter than one pair's latency chain, all four (two pairs
-// taking stages in turn), the first pair draining the accumulator as well.
+// epilogue warps; with the smaller tiles, whose stages are shorter than one task's latency chain, all four (taking whole
+// stages in turn), the first two draining the accumulator as well.
 constexpr int kWorkerGroups = 4;
 constexpr int kWProducerWarp = 2 + 4 * kWorkerGroups;
 constexpr int kTcThreads = 32 * (kWProducerWarp + 1);
@@ -120,9 +123,11 @@ __device__ __forceinline__ uint32_t pack_halves(uint32_t lo, uint32_t hi)
 }
 
 template <int TOK>
-__global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant__ CUtensorMap x_map, const TcParams p)
+__global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map,
+                                                           const __grid_constant__ CUtensorMap zs_map, const TcParams p)
 {
     using Cfg = TcCfg<TOK>;
+    constexpr bool kWhole = TOK < 256;                        // stages move whole: one activation copy, one dequantiser task per quarter
     constexpr int S = Cfg::kStages, SW = Cfg::kWStages;
     extern __shared__ unsigned char smem_raw[];
 
@@ -147,9 +152,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) {
             mbar_init(xfull_bar(2 * s), 1); mbar_init(xfull_bar(2 * s + 1), 1);
-            mbar_init(afull_bar(s), 8); mbar_init(consumed_bar(s), 1); mbar_init(xhalf_bar(s), 1);
+            mbar_init(afull_bar(s), kWhole ? 4 : 8); mbar_init(consumed_bar(s), 1); mbar_init(xhalf_bar(s), 1);
         }
-        for (int s = 0; s < SW; ++s) { mbar_init(wfull_bar(s), 1); mbar_init(wempty_bar(s), 8); }
+        for (int s = 0; s < SW; ++s) { mbar_init(wfull_bar(s), 1); mbar_init(wempty_bar(s), kWhole ? 4 : 8); }
         mbar_init(dfull_bar, 1);
         mbar_init(dempty_bar, 8);
         mbar_init(epi_bar, 8);
@@ -166,9 +171,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
-    const int n_tiles = p.N / kTileN;
-    const int k_steps = (p.K + kBlockK - 1) / kBlockK;        // K % 128 == 64: the last stage carries one 64-k half
-    const bool k_tail = (p.K % kBlockK) != 0;
+    // K % 128 == 64: the last stage carries one 64-k half.  Copies past K, N or the tokens arrive as zeros: codes, zero
+    // points and scales of zero dequantise to zero, so neither edge needs code of its own.
+    const int k_steps = (p.K + kBlockK - 1) / kBlockK;
     const int total_tiles = p.n_blocks * p.t_blocks * p.split;      // work items: (output tile, K part)
     auto k_range = [&](int item, int& ks0, int& ks1) {
         const int kp = item % p.split;
@@ -196,6 +201,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
                     // the middle of the stage's MMAs): each refill starts half a stage earlier than a whole-stage
                     // release would allow
                     const uint32_t dst = smem_base + st * Cfg::kXBytes;
+                    if constexpr (kWhole) {
+                        ok = mbar_wait(consumed_bar(st), phase ^ 1u, abort_flag, kWaitBudgetNs);
+                        if (!ok) break;
+                        mbar_arrive_expect_tx(xfull_bar(2 * st), Cfg::kXBytes);
+                        tma_load_3d(dst, &x_map, 0, tb * TOK, 2 * ks, xfull_bar(2 * st));
+                        if (++st == S) { st = 0; phase ^= 1u; }
+                        continue;
+                    }
                     ok = mbar_wait(xhalf_bar(st), phase ^ 1u, abort_flag, kWaitBudgetNs);
                     if (!ok) break;
                     mbar_arrive_expect_tx(xfull_bar(2 * st), Cfg::kXSubBytes);
@@ -212,48 +225,29 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
         }
     } else if (warp == kWProducerWarp) {
         // ------------------------------ TMA producer of the packed weights ------------------------------
-        // Three lanes share the copies of a stage (an issued copy holds its thread for about a hundred cycles).  A
-        // copy that completes before lane 0 has armed the barrier only drives its byte count negative for a moment;
-        // the phase cannot complete before lane 0's arrival.
-        if (lane < 3) {
-            int sw = 0; uint32_t wphase = 0;
-            bool ok = true;
-            const uint32_t row_words = (uint32_t)n_tiles * 32u;                 // uint4 per k-tile row of the packed matrix
-            const int zs_rows = kBlockK / p.g;                                  // 1 (g = 128) or 2 (g = 64) per stage
-            for (int item = blockIdx.x; item < total_tiles && ok; item += gridDim.x) {
-                const int nb = (item / p.split) % p.n_blocks;
-                const int nb_tiles = min(4, n_tiles - nb * 4);
-                int ks0, ks1;
-                k_range(item, ks0, ks1);
-                const uint32_t w_bytes = nb_tiles * 512u, zs_bytes = nb_tiles * 128u;
-                const uint4* wsrc = p.qw + (size_t)(ks0 * 4) * row_words + nb * 4 * 32;
-                const uint32_t* zsrc = p.zs + (size_t)(ks0 * zs_rows) * p.N + nb * kBlockN;
-                for (int ks = ks0; ks < ks1; ++ks) {
-                    ok = mbar_wait(wempty_bar(sw), wphase ^ 1u, abort_flag, kWaitBudgetNs);
-                    if (!ok) break;
-                    const uint32_t dst = smem_base + Cfg::kWRingOff + sw * Cfg::kWStageBytes;
-                    const uint32_t bar = wfull_bar(sw);
-                    const bool tail = k_tail && ks == k_steps - 1;                  // only the first half exists (g = 64)
-                    if (lane == 0) {
-                        mbar_arrive_expect_tx(bar, tail ? 2 * w_bytes + zs_bytes : 4 * w_bytes + zs_rows * zs_bytes);
-                        bulk_load(dst, wsrc, w_bytes, bar);
-                        bulk_load(dst + 2048, wsrc + row_words, w_bytes, bar);
-                    } else if (lane == 1) {
-                        if (!tail) {
-                            bulk_load(dst + 4096, wsrc + 2 * row_words, w_bytes, bar);
-                            bulk_load(dst + 6144, wsrc + 3 * row_words, w_bytes, bar);
-                        }
-                    } else {
-                        bulk_load(dst + Cfg::kWBytes, zsrc, zs_bytes, bar);
-                        if (zs_rows == 2 && !tail) bulk_load(dst + Cfg::kWBytes + 512, zsrc + p.N, zs_bytes, bar);
-                    }
-                    wsrc += 4 * row_words;
-                    zsrc += (size_t)zs_rows * p.N;
-                    if (++sw == SW) { sw = 0; wphase ^= 1u; }
+        // One tensor copy of the stage's four k-tile rows of four packed tiles and one of its (zero, scale) rows.  (Six
+        // bulk copies shared by three lanes kept this warp busy for about 900 cycles a stage: diverged lanes take turns.)
+        int sw = 0; uint32_t wphase = 0;
+        bool ok = true;
+        const int zs_rows = kBlockK / p.g;                                      // 1 (g = 128) or 2 (g = 64) per stage
+        for (int item = blockIdx.x; item < total_tiles && ok; item += gridDim.x) {
+            const int nb = (item / p.split) % p.n_blocks;
+            int ks0, ks1;
+            k_range(item, ks0, ks1);
+            for (int ks = ks0; ks < ks1; ++ks) {
+                ok = __all_sync(0xffffffffu, mbar_wait(wempty_bar(sw), wphase ^ 1u, abort_flag, kWaitBudgetNs));
+                if (!ok) break;
+                if (elect_one()) {
+                    const uint32_t dst = smem_base + Cfg::kWRingOff + sw * Cfg::kWStageBytes, bar = wfull_bar(sw);
+                    mbar_arrive_expect_tx(bar, Cfg::kWBytes + zs_rows * 512);
+                    tma_load_2d(dst, &w_map, nb * 256, ks * 4, bar);
+                    tma_load_2d(dst + Cfg::kWBytes, &zs_map, nb * kBlockN, ks * zs_rows, bar);
                 }
+                __syncwarp();
+                if (++sw == SW) { sw = 0; wphase ^= 1u; }
             }
-            if (!ok && lane == 0) drain_copies();
         }
+        if (!ok) drain_copies();
     } else if (warp == 5) {
         // ------------------------------ MMA issuer ------------------------------
         // The whole warp walks the loop and an elected lane issues, so that descriptors and addresses stay in uniform
@@ -306,6 +300,21 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
                 const uint32_t a_tmem = tmem_base + Cfg::kACol + 64 * st;
                 const int cur = st;
                 const uint32_t cur_phase = phase;
+                if constexpr (kWhole) {
+                    if (++st == S) { st = 0; phase ^= 1u; }
+                    const bool next_a = mbar_test_wait(afull_bar(st), phase);
+                    const bool next_x = mbar_test_wait(xfull_bar(2 * st), phase);
+                    if (elect_one()) {
+#pragma unroll
+                        for (int kk = 0; kk < 8; ++kk)
+                            mma_f16_ts(tmem_base, a_tmem + 8 * kk, bdesc + (uint64_t)((kk >= 4 ? Cfg::kXSubBytes >> 4 : 0) + 2 * (kk & 3)), idesc,
+                                       ((ks - ks0) | kk) != 0);
+                        tc_commit(consumed_bar(cur));
+                    }
+                    __syncwarp();
+                    ready = __all_sync(0xffffffffu, next_a && next_x);
+                    continue;
+                }
                 // first 64-k half: its activation sub-tile is released by a commit of its own
                 const bool second_x = mbar_test_wait(xfull_bar(2 * cur + 1), cur_phase);
                 if (elect_one()) {
@@ -355,8 +364,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
     } else {
         // ------------------------------ dequant + epilogue (the worker warps) ------------------------------
         // Groups of four warps; a warp may only touch the TMEM lane quarter (warp index % 4), which is also the
-        // packed tile column it dequantises.  Group g takes the g-th 64-k half of every stage: a half keeps a warp
-        // busy for a chain of dependent latencies (shared-memory load, unpack, sub/mul, tcgen05.st, its completion),
+        // packed tile column it dequantises.  With the 256-token tile group g takes the g-th 64-k half of every stage, with
+        // the smaller ones every fourth stage whole: a task keeps a warp busy for a chain of dependent latencies (shared-memory load, unpack, sub/mul, tcgen05.st, its completion),
         // which the ring depth covers.  Two groups drain the accumulator (half of the columns each): with the
         // 256-token tile groups of their own, so that the dequantisers run on into the next tile (its first stages are
         // ready when the accumulator is free again), otherwise the first pair.
@@ -368,8 +377,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
         const int quarter = warp & 3;
         const int wgroup = warp < 4 ? 0 : (warp - 2) / 4;              // 0 .. kWorkerGroups-1
         const int dgroup = wgroup & 1;                                 // which 64-k half of a stage / half of the accumulator's columns
-        const int turn = wgroup >> 1;                                  // GROUPS == 4: which stages (even / odd)
-        uint32_t step_mod = 0;
+        uint32_t step = 0;
         uint32_t epi_phase = 0;
         // bounded rendezvous of the eight dequant/epilogue warps (split-K finalisation)
         auto epi_sync = [&]() -> bool {
@@ -380,7 +388,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
             return done;
         };
         const uint32_t lane_field = (uint32_t)(quarter * 32) << 16;
-        const int zs_row = p.g == 64 ? dgroup : 0;                     // (zero, scale) row of this group's half
         // the epilogue of one work item: drains the accumulator (half of the columns per group), false = a wait gave up
         auto epilogue = [&](int item) -> bool {
             const int tile = item / p.split, kp = item % p.split;
@@ -567,41 +574,46 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
             for (int item = blockIdx.x; item < total_tiles && ok; item += gridDim.x) ok = epilogue(item);
         }
         for (int item = blockIdx.x; item < dequant_tiles && ok; item += gridDim.x) {
-            const int nb = (item / p.split) % p.n_blocks;
-            const bool has_tile = nb * 4 + quarter < n_tiles;
             int ks0, ks1;
             k_range(item, ks0, ks1);
-            for (int ks = ks0; ks < ks1; ++ks, step_mod ^= 1u) {
-                if (GROUPS == 4 && step_mod != (uint32_t)turn) {               // the other pair's stage
+            for (int ks = ks0; ks < ks1; ++ks, ++step) {
+                if (kWhole && (step & 3u) != (uint32_t)wgroup) {               // another set's stage
                     if (++sw == SW) { sw = 0; wphase ^= 1u; }
                     if (++st == S) { st = 0; phase ^= 1u; }
                     continue;
                 }
                 ok = __all_sync(0xffffffffu, mbar_wait(wfull_bar(sw), wphase, abort_flag, kWaitBudgetNs));
                 if (!ok) break;
+                // a task: kHalves 64-k halves of this warp's packed tile column
+                constexpr int kHalves = kWhole ? 2 : 1;
+                const int first = kWhole ? 0 : dgroup;
                 const unsigned char* wst = smem + Cfg::kWRingOff + sw * Cfg::kWStageBytes;
-                const uint4* wq = reinterpret_cast<const uint4*>(wst) + dgroup * 256;
-                const uint32_t* zsp = reinterpret_cast<const uint32_t*>(wst + Cfg::kWBytes + zs_row * 512) + quarter * 32 + r;
-                uint4 q0 = make_uint4(0, 0, 0, 0), q1 = q0;
-                uint32_t zsw[4] = {0, 0, 0, 0};
-                // a missing second half (K % 128 == 64) dequantises to zeros: codes 0 with zero point and scale 0
-                if (has_tile && !(dgroup == 1 && k_tail && ks == k_steps - 1)) {
-                    q0 = wq[quarter * 32 + lane]; q1 = wq[128 + quarter * 32 + lane];
+                const uint4* wq = reinterpret_cast<const uint4*>(wst) + first * 256 + quarter * 32 + lane;
+                uint4 q[2 * kHalves];
+                uint32_t zsw[kHalves][4];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) zsw[j] = zsp[8 * j];
+                for (int i = 0; i < 2 * kHalves; ++i) q[i] = wq[128 * i];
+#pragma unroll
+                for (int half = 0; half < kHalves; ++half) {
+                    const int zs_row = p.g == 64 ? first + half : 0;
+                    const uint32_t* zsp = reinterpret_cast<const uint32_t*>(wst + Cfg::kWBytes + zs_row * 512) + quarter * 32 + r;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) zsw[half][j] = zsp[8 * j];
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(wempty_bar(sw));                // the words are in registers: the stage may refill
                 ok = __all_sync(0xffffffffu, mbar_wait(consumed_bar(st), phase ^ 1u, abort_flag, kWaitBudgetNs));
                 if (!ok) break;
-                if (has_tile) {
-                    tc_fence_after_sync();
-                    const uint32_t words[2][4] = {{q0.x, q0.y, q0.z, q0.w}, {q1.x, q1.y, q1.z, q1.w}};
+                tc_fence_after_sync();
+#pragma unroll
+                for (int half = 0; half < kHalves; ++half) {
+                    const uint32_t words[2][4] = {{q[2 * half].x, q[2 * half].y, q[2 * half].z, q[2 * half].w},
+                                                  {q[2 * half + 1].x, q[2 * half + 1].y, q[2 * half + 1].z, q[2 * half + 1].w}};
 #pragma unroll
                     for (int nh = 0; nh < 2; ++nh) {
                         uint32_t z0, s0, z1, s1;
-                        split_zs(zsw[nh * 2], z0, s0);
-                        split_zs(zsw[nh * 2 + 1], z1, s1);
+                        split_zs(zsw[half][nh * 2], z0, s0);
+                        split_zs(zsw[half][nh * 2 + 1], z1, s1);
                         uint32_t a[16];
 #pragma unroll
                         for (int j = 0; j < 2; ++j)
@@ -615,10 +627,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
                                 d[2] = dequant_h2(h[2], z0, s0);
                                 d[3] = dequant_h2(h[3], z1, s1);
                             }
-                        tmem_st_16x128b_x8(tmem_base + lane_field + ((uint32_t)(nh * 16) << 16) + Cfg::kACol + 64 * st + 32 * dgroup, a);
+                        tmem_st_16x128b_x8(tmem_base + lane_field + ((uint32_t)(nh * 16) << 16) + Cfg::kACol + 64 * st + 32 * (first + half), a);
                     }
-                    tmem_wait_st();
                 }
+                tmem_wait_st();
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(afull_bar(st));
@@ -681,8 +693,8 @@ long long* g_tc_account = nullptr;
 struct TcPlan { int tok, split; };
 
 // Token tile and K split by a cost model in SM clocks, fitted to measurements on B200: a work item costs
-// k-steps x step + epilogue, where a 128-k step costs the larger of its tensor time (4 x tokens) and the issue time of
-// its eight MMAs and one commit, items run in waves of one per SM, and split-K adds the round trip of the fp32
+// k-steps x step + epilogue, where a 128-k step costs 1024 with 256 tokens (tensor time) and 750 with 128 or 64 (700 to 950
+// measured, from half the SMs busy to all; about 1000 before their stages moved whole), items run in waves of one per SM, and split-K adds the round trip of the fp32
 // partial tiles through L2/HBM at about 650 bytes per clock.
 TcPlan pick_plan(int tokens, int N, int K, bool allow_split, int force_split = 0)
 {
@@ -701,8 +713,7 @@ TcPlan pick_plan(int tokens, int N, int K, bool allow_split, int force_split = 0
             if (force_split && sp != force_split) continue;
             const long long items = (long long)n_blocks * ((tokens + t - 1) / t) * sp;
             const long long waves = (items + 147) / 148;
-            const double issue = 8 * 94.0 + 205.0 + 60.0;           // eight MMAs, one commit, the loop around them
-            const double step = 4.0 * t > issue ? 4.0 * t : issue;
+            const double step = t == 256 ? 1024.0 : 750.0;          // the small tiles' pace is that of their producers and dequantisers
             double cost = waves * ((double)(k_steps / sp) * step + 6.0 * t + 2000);
             if (sp > 1) cost += (double)sp * tokens * N * 8.0 / 650.0 + 3000;        // partials written + read back
             if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = {t, sp}; }
@@ -717,7 +728,7 @@ size_t split_workspace_bytes(int tokens, int N, int split, int tiles)
 }
 
 template <int TOK>
-int launch_tok(const CUtensorMap& map, const TcParams& p, int grid, cudaStream_t st)
+int launch_tok(const CUtensorMap& map, const CUtensorMap& w_map, const CUtensorMap& zs_map, const TcParams& p, int grid, cudaStream_t st)
 {
     static int configured[64] = {0};
     int dev = 0;
@@ -728,7 +739,7 @@ int launch_tok(const CUtensorMap& map, const TcParams& p, int grid, cudaStream_t
         if (e != cudaSuccess) return record_cuda_error(e);
         if (dev < 64) configured[dev] = 1;
     }
-    tc_kernel<TOK><<<grid, kTcThreads, TcCfg<TOK>::kSmemBytes, st>>>(map, p);
+    tc_kernel<TOK><<<grid, kTcThreads, TcCfg<TOK>::kSmemBytes, st>>>(map, w_map, zs_map, p);
     count_launch();
     e = cudaGetLastError();
     return e == cudaSuccess ? W4A16_OK : record_cuda_error(e);
@@ -761,11 +772,28 @@ int launch_tc(const GemmArgs& a, void* workspace, size_t workspace_bytes, cudaSt
     TcPlan pl = pick_plan(a.tokens, a.N, a.K, workspace != nullptr, force_split);
     const int tok = pl.tok;
 
-    CUtensorMap map;
-    {
+    CUtensorMap map, w_map, zs_map;
+    if (tok == 256) {
         const uint64_t dims[2] = {(uint64_t)a.K, (uint64_t)a.tokens};
         const uint32_t box[2] = {(uint32_t)kSubK, (uint32_t)tok};
         int s = encode_tensor_map_2d(&map, a.x, 2, dims, (uint64_t)a.K * sizeof(__half), box, /*swizzle128*/ true);
+        if (s != W4A16_OK) return s;
+    } else {
+        // as [K/64][tokens][64]: a box of two is a stage's two swizzled sub-tiles, one copy
+        const uint64_t dims[3] = {(uint64_t)kSubK, (uint64_t)a.tokens, (uint64_t)(a.K / kSubK)}, strides[2] = {(uint64_t)a.K * sizeof(__half), kSubK * sizeof(__half)};
+        const uint32_t box[3] = {(uint32_t)kSubK, (uint32_t)tok, 2};
+        int s = encode_tensor_map(&map, a.x, 2, 3, dims, strides, box, /*swizzle128*/ true);
+        if (s != W4A16_OK) return s;
+    }
+    {
+        // the packed matrix as 64-bit words, one row per k-tile row
+        const uint64_t row_bytes = (uint64_t)(a.N / kTileN) * 512, dims[2] = {row_bytes / 8, (uint64_t)(a.K / kTileK)};
+        const uint32_t box[2] = {256, 4};
+        int s = encode_tensor_map_2d(&w_map, a.qw, 8, dims, row_bytes, box, /*swizzle128*/ false);
+        if (s != W4A16_OK) return s;
+        const uint64_t zdims[2] = {(uint64_t)a.N, (uint64_t)(a.K / a.g)};
+        const uint32_t zbox[2] = {(uint32_t)kBlockN, (uint32_t)(kBlockK / a.g)};
+        s = encode_tensor_map_2d(&zs_map, a.zs, 4, zdims, (uint64_t)a.N * 4, zbox, /*swizzle128*/ false);
         if (s != W4A16_OK) return s;
     }
 
@@ -797,9 +825,9 @@ int launch_tc(const GemmArgs& a, void* workspace, size_t workspace_bytes, cudaSt
     const long long items = tiles * pl.split;
     const int grid = (int)(items < sms ? items : sms);
     switch (tok) {
-        case 256: return launch_tok<256>(map, p, grid, st);
-        case 128: return launch_tok<128>(map, p, grid, st);
-        default:  return launch_tok<64>(map, p, grid, st);
+        case 256: return launch_tok<256>(map, w_map, zs_map, p, grid, st);
+        case 128: return launch_tok<128>(map, w_map, zs_map, p, grid, st);
+        default:  return launch_tok<64>(map, w_map, zs_map, p, grid, st);
     }
 }
 
