@@ -122,6 +122,26 @@ def _stream(t: torch.Tensor) -> int:
     return torch.cuda.current_stream(t.device).cuda_stream
 
 
+def _half_like(t, device: int, numel: int) -> bool:
+    """A contiguous fp16 CUDA tensor of `numel` elements on CUDA device `device`."""
+    return isinstance(t, torch.Tensor) and t.is_cuda and t.dtype == torch.float16 and t.get_device() == device and \
+        t.numel() == numel and t.is_contiguous()
+
+
+def _plain_call(I, W, ZS, bias, N, g, residual):
+    """Whether these are correct arguments of a plain linear on the current device: every check of gemm_awq_bias in one
+    pass.  An eager call of a small linear is host time (4096 x 4096, one token: the kernel runs 5 us), and the checks
+    with their messages, the device guard and the stream object took more of it than the launch."""
+    if not (isinstance(I, torch.Tensor) and isinstance(W, torch.Tensor) and I.is_cuda and W.is_cuda and I.dim() == 3 and W.dim() == 2 and
+            I.dtype == torch.float16 and I.is_contiguous() and W.is_contiguous() and g > 0 and N > 0):
+        return False
+    b, s, K = I.shape
+    dev = I.get_device()
+    return (K % g == 0 and W.get_device() == dev and W.numel() * W.element_size() * 2 == K * N and _half_like(ZS, dev, K // g * N * 2) and
+            ZS.dim() == 2 and (bias is None or _half_like(bias, dev, N)) and (residual is None or _half_like(residual, dev, b * s * N)) and
+            torch.cuda.current_device() == dev)
+
+
 def _need(cond: bool, msg: str) -> None:
     if not cond:
         raise RuntimeError(msg)
@@ -178,12 +198,32 @@ def gemm_awq_bias(I, W, W_zeros_scales, bias, N: int, group_size: int, algo: int
     row_stats_buffer the GEMV that produced I filled (stats_out=...), or None: the normalisation then runs as its own
     launch.  stats_out: leave the row statistics of this call's output there (up to 16 tokens; ignored beyond).
     """
+    N = int(N)
+    group_size = int(group_size)
+    if pre_norm is None and stats_out is None and out is None and \
+            _plain_call(I, W, W_zeros_scales, bias, N, group_size, residual):
+        b, s, K = I.shape
+        tokens, dev = b * s, I.get_device()
+        lib = _lib or load_library()
+        out = I.new_empty((b, s, N // 2 if silu_mul else N))
+        ws, ws_bytes = None, 0
+        if tokens > 32:                                      # none below (w4a16_workspace_bytes)
+            ws_bytes = lib.w4a16_workspace_bytes(tokens, N, K, group_size)
+            if ws_bytes:
+                ws = torch.empty(ws_bytes, dtype=torch.uint8, device=I.device)
+        st = lib.w4a16_gemm_fused(I.data_ptr(), W.data_ptr(), W_zeros_scales.data_ptr(), None if bias is None else bias.data_ptr(),
+                                  None if residual is None else residual.data_ptr(), out.data_ptr(), tokens, N, K, group_size,
+                                  None if ws is None else ws.data_ptr(), ws_bytes, torch._C._cuda_getCurrentRawStream(dev), int(algo),
+                                  (FLAG_STATIC_WEIGHTS if static_weights else 0) | (FLAG_RELU if relu else 0) |
+                                  (FLAG_SILU_MUL if silu_mul else 0))
+        if st:
+            _check(st, "gemm_awq_ut")
+        return out
+    # anything else: the checks one by one, each with its message
     _check_tensor(I, "I", dtype=torch.float16, dims=3)
     _check_tensor(W, "W", dims=2)
     _check_tensor(W_zeros_scales, "W_zeros_scales", dtype=torch.float16, dims=2)
     b, s, K = I.shape
-    N = int(N)
-    group_size = int(group_size)
     _need(W.device == I.device and W_zeros_scales.device == I.device, "all tensors must be on the same device")
     _need(group_size > 0 and N > 0, "unsupported group size" if group_size <= 0 else "N must be positive")
     _need(W.numel() * W.element_size() * 2 == K * N, f"Tensor W must hold K*N/2 = {K * N // 2} bytes of packed int4")
