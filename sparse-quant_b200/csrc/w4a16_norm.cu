@@ -14,7 +14,7 @@ namespace w4a16 {
 namespace {
 
 constexpr int kNormThreads = 256;
-constexpr int kNormMaxVec = 4;                 // 16-byte vectors per thread: rows of up to 256 * 4 * 8 = 8192 halfs
+constexpr int kNormMaxVec = 4;                 // most 16-byte vectors per thread: rows of up to 256 * 4 * 8 = 8192 halfs
 
 struct NormParams {
     const __half* x;
@@ -42,6 +42,11 @@ __device__ __forceinline__ float block_sum(float v, float* scratch)
     return s;
 }
 
+// NV = 16-byte vectors per thread (1, 2 or 4, the fewest that cover a row).  A row is a chain of latencies: load, one or two
+// CTA-wide sums, store.  The affine parameters depend on nothing in that chain and are requested before it (they used to
+// be loaded behind the sums, another trip to memory): 8 rows of 4096 4.7 -> 3.9 us (LayerNorm), 32 rows 3.4 -> 2.6 us
+// (RMSNorm), 4096 rows 17.6 -> 15.9 us.
+template <int NV>
 __global__ void __launch_bounds__(kNormThreads) add_norm_kernel(const NormParams p)
 {
     __shared__ float scratch[kNormThreads / 32];
@@ -52,10 +57,20 @@ __global__ void __launch_bounds__(kNormThreads) add_norm_kernel(const NormParams
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const size_t row = (size_t)blockIdx.x * p.cols;
     const int nvec = p.cols / 8;
-    float v[kNormMaxVec][8];
+    uint4 wv[NV], bv[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int c = threadIdx.x + i * kNormThreads;
+        wv[i] = bv[i] = make_uint4(0, 0, 0, 0);
+        if (c < nvec) {
+            wv[i] = *reinterpret_cast<const uint4*>(p.weight + c * 8);
+            if (p.bias) bv[i] = *reinterpret_cast<const uint4*>(p.bias + c * 8);
+        }
+    }
+    float v[NV][8];
     float sum = 0.f;
 #pragma unroll
-    for (int i = 0; i < kNormMaxVec; ++i) {
+    for (int i = 0; i < NV; ++i) {
         const int c = threadIdx.x + i * kNormThreads;
         if (c < nvec) {
             uint4 a = *reinterpret_cast<const uint4*>(p.x + row + c * 8);
@@ -84,7 +99,7 @@ __global__ void __launch_bounds__(kNormThreads) add_norm_kernel(const NormParams
         mean = sum / p.cols;
         float sq = 0.f;
 #pragma unroll
-        for (int i = 0; i < kNormMaxVec; ++i)
+        for (int i = 0; i < NV; ++i)
             if (threadIdx.x + i * kNormThreads < nvec)
 #pragma unroll
                 for (int e = 0; e < 8; ++e) sq += (v[i][e] - mean) * (v[i][e] - mean);
@@ -92,14 +107,11 @@ __global__ void __launch_bounds__(kNormThreads) add_norm_kernel(const NormParams
         rstd = rsqrtf(sq / p.cols + p.eps);
     }
 #pragma unroll
-    for (int i = 0; i < kNormMaxVec; ++i) {
+    for (int i = 0; i < NV; ++i) {
         const int c = threadIdx.x + i * kNormThreads;
         if (c < nvec) {
-            const uint4 w = *reinterpret_cast<const uint4*>(p.weight + c * 8);
-            const __half* wh = reinterpret_cast<const __half*>(&w);
-            uint4 b = make_uint4(0, 0, 0, 0);
-            if (p.bias) b = *reinterpret_cast<const uint4*>(p.bias + c * 8);
-            const __half* bh = reinterpret_cast<const __half*>(&b);
+            const __half* wh = reinterpret_cast<const __half*>(&wv[i]);
+            const __half* bh = reinterpret_cast<const __half*>(&bv[i]);
             uint4 o;
             __half* oh = reinterpret_cast<__half*>(&o);
 #pragma unroll
@@ -206,7 +218,8 @@ extern "C" int w4a16_add_norm(const void* x, const void* delta, void* x_out, voi
     NormParams p;
     p.x = (const __half*)x; p.delta = (const __half*)delta; p.x_out = (__half*)x_out; p.h_out = (__half*)h_out;
     p.weight = (const __half*)weight; p.bias = (const __half*)bias; p.cols = cols; p.eps = eps; p.rms = rms ? 1 : 0;
-    cudaError_t e = launch_after_previous(add_norm_kernel, dim3(rows), dim3(kNormThreads), 0, (cudaStream_t)stream, p);
+    auto kernel = cols <= kNormThreads * 8 ? add_norm_kernel<1> : cols <= kNormThreads * 16 ? add_norm_kernel<2> : add_norm_kernel<4>;
+    cudaError_t e = launch_after_previous(kernel, dim3(rows), dim3(kNormThreads), 0, (cudaStream_t)stream, p);
     count_launch();
     return e == cudaSuccess ? W4A16_OK : record_cuda_error(e);
 }
