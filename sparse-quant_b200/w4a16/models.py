@@ -235,10 +235,10 @@ def _layer_forward_static(self, x, pos_t, rope, stats=None):
         a = decode_attention(qkv, self.k_cache, self.v_cache, pos_t, self.local_heads, rope=rope).view(B, 1, -1)
         x, h = add_norm(x, self.out_proj(a), *_norm_args(self.ln2))
         if self.cfg.kind == "opt":
-            return x + self.fc2(self.fc1(h.reshape(1, B, H), relu=True)).reshape(B, 1, H)
+            return self.fc2(self.fc1(h.reshape(1, B, H), relu=True), residual=x.reshape(1, B, H)).reshape(B, 1, H)
         if B <= 32:
-            return x + self.fc2(self.gate_up_proj(h, silu_mul=True))
-        return x + self.fc2(silu_mul_tiles(self.gate_up_proj(h)))
+            return self.fc2(self.gate_up_proj(h, silu_mul=True), residual=x)
+        return self.fc2(silu_mul_tiles(self.gate_up_proj(h)), residual=x)
     s_in, s_mid, s_out = stats
     qkv = self.qkv_proj(x, pre_norm=(*_norm_args(self.ln1), s_in)).view(B, -1)
     a = decode_attention(qkv, self.k_cache, self.v_cache, pos_t, self.local_heads, rope=rope).view(B, 1, -1)
