@@ -182,7 +182,7 @@ extern "C" int w4a16_gemm_fused(const void* x, const void* qweight, const void* 
     int s = validate(x, qweight, zeros_scales, out, tokens, N, K, group_size);
     if (s != W4A16_OK) return s;
     if (algo != W4A16_ALGO_AUTO && algo != W4A16_ALGO_SKINNY && algo != W4A16_ALGO_TC) return W4A16_ERR_BAD_ALGO;
-    if (flags & ~(unsigned)(W4A16_FLAG_STATIC_WEIGHTS | W4A16_FLAG_RELU | W4A16_FLAG_SILU_MUL)) return W4A16_ERR_BAD_ALGO;
+    if (flags & ~(unsigned)(W4A16_FLAG_STATIC_WEIGHTS | W4A16_FLAG_RELU | W4A16_FLAG_SILU_MUL | W4A16_FLAG_RELU_KEEPS_NAN)) return W4A16_ERR_BAD_ALGO;
     if (tokens == 0) return W4A16_OK;
     if (residual && ((uintptr_t)residual & 1)) return W4A16_ERR_MISALIGNED;
     s = check_device();
@@ -195,6 +195,7 @@ extern "C" int w4a16_gemm_fused(const void* x, const void* qweight, const void* 
     a.static_weights = (flags & W4A16_FLAG_STATIC_WEIGHTS) != 0;
     a.relu = (flags & W4A16_FLAG_RELU) != 0;
     a.silu_mul = (flags & W4A16_FLAG_SILU_MUL) != 0;
+    a.relu_keeps_nan = (flags & W4A16_FLAG_RELU_KEEPS_NAN) != 0;
 
     const int forced = decode_forced_kernel();
     const bool narrow = forced == 3 ? algo != W4A16_ALGO_TC && narrow_supported(tokens, N, K, group_size)
@@ -205,7 +206,13 @@ extern "C" int w4a16_gemm_fused(const void* x, const void* qweight, const void* 
         // w4a16_silu_mul on the plain output
         if (algo != W4A16_ALGO_SKINNY || tokens > 32 || (N % 64) || residual) return W4A16_ERR_BAD_ALGO;
     }
+    if (a.relu_keeps_nan && (narrow || algo != W4A16_ALGO_TC)) return W4A16_ERR_BAD_ALGO;
     if (narrow) {
+        // beyond 32 tokens a workspace is checked as for the kernel that would use it: one too small is an error either way
+        if (tokens > 32 && workspace) {
+            if (workspace_bytes < tc_workspace_bytes(tokens, N, K, group_size)) return W4A16_ERR_WORKSPACE;
+            if (tc_workspace_bytes(tokens, N, K, group_size) && ((uintptr_t)workspace & 255)) return W4A16_ERR_MISALIGNED;
+        }
         s = launch_narrow(a, (cudaStream_t)stream);
         if (s != W4A16_ERR_BAD_ALGO || forced == 3) return s;         // no launch shape: the kernels below
     }

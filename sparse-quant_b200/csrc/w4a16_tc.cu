@@ -105,7 +105,7 @@ struct TcParams {
     int*            error;          // device word, set non-zero on a wait timeout
     int tokens, N, K, g;
     int n_blocks, t_blocks;
-    int relu;                       // clamp the outputs at zero after the bias add
+    int relu;                       // clamp the outputs at zero after the bias add (2: NaN stays NaN)
     const __half* residual;         // [tokens, N] added after bias / ReLU (fp16 add), or null
     int split;                      // K parts per output tile (1 = no split)
     float* partial;                 // split > 1: fp32 partial tiles [split][tokens][N]
@@ -450,9 +450,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
                         __half2 o[4];
 #pragma unroll
                         for (int j = 0; j < 4; ++j) o[j] = __hadd2(*reinterpret_cast<__half2*>(&h[i + j]), bias2);
-                        if (p.relu) {
+                        if (p.relu == 1) {
 #pragma unroll
                             for (int j = 0; j < 4; ++j) o[j] = __hmax2(o[j], __half2half2(__half()));
+                        } else if (p.relu) {
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) o[j] = __hmax2_nan(o[j], __half2half2(__half()));
                         }
                         if (p.residual) {
                             __half r[8];
@@ -500,7 +503,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
             }
             auto finish = [&](float acc, int t) {                                // one output element
                 __half h = __hadd(__float2half_rn(acc), bias);
-                if (p.relu) h = __hmax(h, __half());
+                if (p.relu) h = p.relu == 2 ? __hmax_nan(h, __half()) : __hmax(h, __half());
                 if (p.residual) h = __hadd(h, p.residual[(size_t)t * p.N + n]);
                 p.out[(size_t)t * p.N + n] = h;
             };
@@ -799,7 +802,7 @@ int launch_tc(const GemmArgs& a, void* workspace, size_t workspace_bytes, cudaSt
 
     TcParams p;
     p.qw = reinterpret_cast<const uint4*>(a.qw); p.zs = a.zs; p.bias = a.bias; p.out = a.out; p.error = err;
-    p.tokens = a.tokens; p.N = a.N; p.K = a.K; p.g = a.g; p.relu = a.relu ? 1 : 0; p.residual = a.residual; p.account = g_tc_account;
+    p.tokens = a.tokens; p.N = a.N; p.K = a.K; p.g = a.g; p.relu = a.relu ? (a.relu_keeps_nan ? 2 : 1) : 0; p.residual = a.residual; p.account = g_tc_account;
     p.n_blocks = (a.N + kBlockN - 1) / kBlockN;
     p.t_blocks = (a.tokens + tok - 1) / tok;
     const long long tiles = (long long)p.n_blocks * p.t_blocks;

@@ -128,6 +128,10 @@ def _half_like(t, device: int, numel: int) -> bool:
         t.numel() == numel and t.is_contiguous()
 
 
+def _relu_flags(relu) -> int:
+    return 0 if not relu else FLAG_RELU | FLAG_RELU_KEEPS_NAN if relu == RELU_KEEPS_NAN else FLAG_RELU
+
+
 def _plain_call(I, W, ZS, bias, N, g, residual):
     """Whether these are correct arguments of a plain linear on the current device: every check of gemm_awq_bias in one
     pass.  An eager call of a small linear is host time (4096 x 4096, one token: the kernel runs 5 us), and the checks
@@ -165,6 +169,8 @@ def launch_count() -> int:
 FLAG_STATIC_WEIGHTS = 1
 FLAG_RELU = 2
 FLAG_SILU_MUL = 4
+FLAG_RELU_KEEPS_NAN = 8
+RELU_KEEPS_NAN = 2        # relu=RELU_KEEPS_NAN: torch.relu's treatment of NaN (prefill kernel only)
 
 
 def prenorm_supported(tokens: int, K: int) -> bool:
@@ -191,7 +197,7 @@ def gemm_awq_bias(I, W, W_zeros_scales, bias, N: int, group_size: int, algo: int
     [K/g, 2N]; bias fp16 with N elements or None.  Returns fp16 [b, s, N].
     static_weights=True passes W4A16_FLAG_STATIC_WEIGHTS (see include/w4a16_b200.h): only for weights
     that were written before anything still in flight on the current stream was enqueued.
-    relu=True passes W4A16_FLAG_RELU: max(., 0) applied after the bias add.
+    relu=True passes W4A16_FLAG_RELU: max(., 0) applied after the bias add (NaN becomes 0; relu=RELU_KEEPS_NAN: stays NaN).
     residual (fp16 [b, s, N]) is added to the output in the kernel epilogue; silu_mul=True passes
     W4A16_FLAG_SILU_MUL (gate / up tiles interleaved, see w4a16_gemm_fused): returns fp16 [b, s, N/2].
     pre_norm = (weight, bias or None, eps, rms, stats): the linear is applied to LayerNorm / RMSNorm of I; `stats` is the
@@ -214,7 +220,7 @@ def gemm_awq_bias(I, W, W_zeros_scales, bias, N: int, group_size: int, algo: int
         st = lib.w4a16_gemm_fused(I.data_ptr(), W.data_ptr(), W_zeros_scales.data_ptr(), None if bias is None else bias.data_ptr(),
                                   None if residual is None else residual.data_ptr(), out.data_ptr(), tokens, N, K, group_size,
                                   None if ws is None else ws.data_ptr(), ws_bytes, torch._C._cuda_getCurrentRawStream(dev), int(algo),
-                                  (FLAG_STATIC_WEIGHTS if static_weights else 0) | (FLAG_RELU if relu else 0) |
+                                  (FLAG_STATIC_WEIGHTS if static_weights else 0) | _relu_flags(relu) |
                                   (FLAG_SILU_MUL if silu_mul else 0))
         if st:
             _check(st, "gemm_awq_ut")
@@ -259,7 +265,7 @@ def gemm_awq_bias(I, W, W_zeros_scales, bias, N: int, group_size: int, algo: int
                                             float(eps), int(bool(rms)), W.data_ptr(), W_zeros_scales.data_ptr(),
                                             bias.data_ptr() if bias is not None else None, out.data_ptr(), tokens, N, K,
                                             group_size, _stream(I),
-                                            (FLAG_STATIC_WEIGHTS if static_weights else 0) | (FLAG_RELU if relu else 0) |
+                                            (FLAG_STATIC_WEIGHTS if static_weights else 0) | _relu_flags(relu) |
                                             (FLAG_SILU_MUL if silu_mul else 0))
             _check(st, "gemm_awq_ut")
             return out
@@ -270,7 +276,7 @@ def gemm_awq_bias(I, W, W_zeros_scales, bias, N: int, group_size: int, algo: int
                                                bias.data_ptr() if bias is not None else None,
                                                residual.data_ptr() if residual is not None else None, out.data_ptr(),
                                                stats_out.data_ptr(), tokens, N, K, group_size, _stream(I),
-                                               (FLAG_STATIC_WEIGHTS if static_weights else 0) | (FLAG_RELU if relu else 0))
+                                               (FLAG_STATIC_WEIGHTS if static_weights else 0) | _relu_flags(relu))
         _check(st, "gemm_awq_ut")
         return out
     with torch.cuda.device(I.device):
@@ -281,7 +287,7 @@ def gemm_awq_bias(I, W, W_zeros_scales, bias, N: int, group_size: int, algo: int
                                   residual.data_ptr() if residual is not None else None, out.data_ptr(),
                                   tokens, N, K, group_size,
                                   ws.data_ptr() if ws is not None else None, ws_bytes, _stream(I), int(algo),
-                                  (FLAG_STATIC_WEIGHTS if static_weights else 0) | (FLAG_RELU if relu else 0) |
+                                  (FLAG_STATIC_WEIGHTS if static_weights else 0) | _relu_flags(relu) |
                                   (FLAG_SILU_MUL if silu_mul else 0))
     _check(st, "gemm_awq_ut")
     return out

@@ -179,7 +179,7 @@ def _layer_forward_kernels(self, x, pos0: int, rope=None):
     one pass over memory each (an OPT-shaped layer of 8 x 512 tokens spent 250 us in torch's elementwise and copy kernels,
     a LLaMA-shaped one of 3 x 333 tokens 350 us, as much as in its linears; a prefill of four layers 6580 -> 5980 us and
     3138 -> 1886 us with them gone)."""
-    from quant import add_norm, append_qkv, silu_mul_tiles
+    from quant import RELU_KEEPS_NAN, add_norm, append_qkv, silu_mul_tiles
     B, S, H = x.shape
     D, heads = self.head_dim, self.local_heads
     # from 256 tokens on the residual and the ReLU go into the linears' epilogues, where they hide behind the next
@@ -200,7 +200,8 @@ def _layer_forward_kernels(self, x, pos0: int, rope=None):
         x, h = add_norm(x, self.out_proj(a), *_norm_args(self.ln2))
     if self.cfg.kind == "opt":
         h = h.reshape(1, B * S, H)
-        f = self.fc1(h, relu=True) if fold else torch.relu(self.fc1(h))
+        # (groups of 32 run in the decode kernels, whose ReLU turns NaN into 0)
+        f = self.fc1(h, relu=RELU_KEEPS_NAN) if fold and self.cfg.group_size != 32 else torch.relu(self.fc1(h))
     else:
         f = silu_mul_tiles(self.gate_up_proj(h))
     if fold:

@@ -54,7 +54,7 @@ class WALinear(nn.Module):
             x3 = x3.contiguous()
         extra = {}
         if relu:
-            extra["relu"] = True
+            extra["relu"] = relu
         if silu_mul:
             extra["silu_mul"] = True
         if residual is not None:

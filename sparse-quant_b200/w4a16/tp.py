@@ -142,7 +142,7 @@ class ColumnParallelWALinear(nn.Module):
     def forward(self, x, relu: bool = False, pre_norm=None):
         extra = {}
         if relu:
-            extra["relu"] = True
+            extra["relu"] = relu
         if pre_norm is not None:
             extra["pre_norm"] = pre_norm
         return self.linear(x, **extra)

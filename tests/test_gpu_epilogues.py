@@ -188,3 +188,21 @@ def test_row_parallel_residual_single_rank_exchange(M):
         parts = int(stats[:1].view(torch.int32).item())
         data = stats[4:4 + parts * 32].view(parts, 16, 2).double().sum(0)[:M].cpu()
         assert torch.allclose(data[:, 0], got[0].double().sum(-1).cpu(), rtol=1e-5, atol=1e-2)
+
+
+def test_relu_epilogue_can_keep_nan():
+    """W4A16_FLAG_RELU_KEEPS_NAN is torch.relu on the plain output, split K included; the other kernels refuse it."""
+    import quant
+    for (M, N, K, g) in [(300, 256, 512, 128), (270, 96, 1344, 64), (40, 256, 8192, 128)]:
+        p = make_packed(N, K, g, seed=5)
+        qw, zs = to_dev(p)
+        x = make_x(M, K, seed=2)
+        x[0, 3, 7] = float("nan")
+        x[0, M - 1, 0] = float("inf")
+        x = x.cuda()
+        plain = quant.gemm_awq_bias(x, qw, zs, None, N, g, algo=quant.ALGO_TC)
+        kept = quant.gemm_awq_bias(x, qw, zs, None, N, g, algo=quant.ALGO_TC, relu=quant.RELU_KEEPS_NAN)
+        assert torch.equal(torch.nan_to_num(kept, nan=-1.0), torch.nan_to_num(torch.relu(plain), nan=-1.0))
+        assert bool(kept[0, 3].isnan().all()) and not bool(quant.gemm_awq_bias(x, qw, zs, None, N, g, algo=quant.ALGO_TC, relu=True).isnan().any())
+    with pytest.raises(RuntimeError):
+        quant.gemm_awq_bias(x[:, :20].contiguous(), qw, zs, None, N, g, relu=quant.RELU_KEEPS_NAN)
