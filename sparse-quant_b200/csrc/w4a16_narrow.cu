@@ -593,8 +593,8 @@ bool narrow_preferred(int tokens, int N, int K, int g)
     // 23.9 / 15.8 (12288), 26.3 / 17.6 (16384), 32.3 / 17.8 (16384 -> 4096), 35.4 / 28.4 (4096 -> 22016, g = 64): from 17 on.
     // At 9 to 16 tokens they are level with groups of 128 (7.4 / 7.8, 14.9 / 14.1, 15.4 / 15.6, 16.6 / 16.6), this one
     // ahead with groups of 64, twice the scale work for them (29.6 / 23.3, 15.8 / 13.5).  At 33 to 64 the prefill kernel's
-    // 64-token tile, which does not split K, leaves SMs idle on all but the widest matrices: 20.6 / 9.7 (4096 -> 4096), 28.8 / 20.3
-    // (11008 -> 4096), 21.0 / 21.6 (4096 -> 12288), 41.2 / 42.8 (22016).
+    // 64-token tile, which does not split a short K, leaves SMs idle on all but the widest matrices: at 48 tokens 16.3 / 9.3
+    // (4096 -> 4096), 26.7 / 20.0 (11008 -> 4096), 30.3 / 20.0 (16384 -> 4096), but 17.1 / 20.3 (4096 -> 12288), 31.2 / 41.2 (22016).
     if (!narrow_supported(tokens, N, K, g)) return false;
     if (tokens > 32) return N < 12288;
     return tokens > (g == 64 ? 8 : 16);
