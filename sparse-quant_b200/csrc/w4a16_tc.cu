@@ -38,8 +38,8 @@
 //   W ring   (shared memory, own depth): the stage's packed weight tiles (a box of four k-tile rows by four tiles,
 //            one tensor copy) and the (zero, scale) row(s), filled by the last warp, read only by the dequantisers and
 //            released as soon as they hold the words in registers.
-//   dequantisers (groups of four; with the 256-token tile a pair of groups takes the two 64-k halves of a stage): read 16 B per lane per 32x32 tile from shared memory, expand the nibbles in
-//            registers, (t - z) * s with
+//   dequantisers (groups of four; with the 256-token tile a pair of groups takes the two 64-k halves of a stage): read
+//            16 B per lane per 32x32 tile from shared memory, expand the nibbles in registers, (t - z) * s with
 //            sub.ftz/mul.ftz (bit-exact with the reference), and write the fp16 result straight into tensor memory
 //            with tcgen05.st.16x128b - the packed layout is already that fragment order - so the dequantised weights
 //            never touch shared memory.
@@ -98,8 +98,6 @@ struct TcCfg {
 };
 
 struct TcParams {
-    const uint4*    qw;
-    const uint32_t* zs;
     const __half*   bias;
     __half*         out;
     int*            error;          // device word, set non-zero on a wait timeout
@@ -801,7 +799,7 @@ int launch_tc(const GemmArgs& a, void* workspace, size_t workspace_bytes, cudaSt
     }
 
     TcParams p;
-    p.qw = reinterpret_cast<const uint4*>(a.qw); p.zs = a.zs; p.bias = a.bias; p.out = a.out; p.error = err;
+    p.bias = a.bias; p.out = a.out; p.error = err;
     p.tokens = a.tokens; p.N = a.N; p.K = a.K; p.g = a.g; p.relu = a.relu ? (a.relu_keeps_nan ? 2 : 1) : 0; p.residual = a.residual; p.account = g_tc_account;
     p.n_blocks = (a.N + kBlockN - 1) / kBlockN;
     p.t_blocks = (a.tokens + tok - 1) / tok;
