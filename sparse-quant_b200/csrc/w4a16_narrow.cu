@@ -48,6 +48,7 @@ constexpr int kBlockN = 128, kBlockK = 128;
 constexpr uint64_t kWaitBudgetNs = 400ull * 1000 * 1000;
 constexpr int kMaxStages = 16;
 constexpr int kFirstDequantWarp = 4, kFirstEpilogueWarp = 20;
+constexpr int kDequantSets = (kFirstEpilogueWarp - kFirstDequantWarp) / 4;      // sets of four warps that take stages in turn
 constexpr int kNarrowSmem = 227 * 1024;
 
 template <int T, int G>
@@ -253,10 +254,21 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
         auto step = [](int& i, int by, int n) { i += by; const bool wrap = i >= n; if (wrap) i -= n; return wrap; };
         int st = set, slot = set % R, freed = set + Q - R; uint32_t phase = 0, freed_phase = 1;    // freed: the stage R back, whose A slot is taken
         if (freed >= Q) { freed -= Q; freed_phase = 0; }
-        for (int it = set; it < total; it += 4) {
+        // A wait names a round of a ring by its parity, which is only right where the round before is known to be complete.
+        // What a set knows of the weights of stage it - Q, which another set unpacked, comes from its own last stage: all
+        // MMAs up to it - 4 - R have run, so the weights up to there had landed.  With fewer than R + 4 stages that does not
+        // reach it - Q: a set that overtook one still waiting for its weights would take those for its own, read them half
+        // landed and hand their slot to the next copy.  There it waits for the MMAs of stage it - Q first.
+        const bool shallow = Q < R + kDequantSets;
+        for (int it = set; it < total; it += kDequantSets) {
             {
-                const bool loaded = mbar_test_wait(wfull_bar(st), phase);            // both probes in flight together
+                const bool turned = !(shallow && it >= Q) || mbar_test_wait(done_bar(st), phase ^ 1u);
+                bool loaded = mbar_test_wait(wfull_bar(st), phase);                  // the probes are in flight together
                 const bool slot_free = it < R || mbar_test_wait(done_bar(freed), freed_phase);
+                if (!__all_sync(0xffffffffu, turned)) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(done_bar(st), phase ^ 1u, abort_flag, kWaitBudgetNs))) break;
+                    loaded = false;                                                  // asked before that round was known to be over
+                }
                 if (!loaded && !mbar_wait(wfull_bar(st), phase, abort_flag, kWaitBudgetNs)) break;    // the same for every lane
                 __syncwarp();
                 const unsigned char* wst = smem + w_off + st * Cfg::kWStage;
@@ -306,9 +318,9 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
                 __syncwarp();
                 if (lane == 0) mbar_arrive(ready_bar(st));
             }
-            if (step(st, 4, Q)) phase ^= 1u;
-            step(slot, 4 % R, R);
-            if (step(freed, 4, Q)) freed_phase ^= 1u;
+            if (step(st, kDequantSets, Q)) phase ^= 1u;
+            step(slot, kDequantSets % R, R);
+            if (step(freed, kDequantSets, Q)) freed_phase ^= 1u;
         }
     } else if (warp >= kFirstEpilogueWarp) {
         // ---- scale and accumulate: thread = out-feature (tensor memory lane), registers = tokens ----

@@ -95,6 +95,9 @@ struct TcCfg {
     static_assert(8 * kBarriers + 12 <= kBarrierBytes, "barrier area");
     static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
     static_assert(kACol + 64 * kStages + (TOK == 256 ? 64 : 0) <= kTmemCols, "TMEM budget");
+    // a wait names a round by its parity: a dequantiser group must know that the stage's round before is over, which it
+    // does where the stage comes back to the same group
+    static_assert(TOK == 256 || kWStages % kWorkerGroups == 0, "a stage of the weight ring belongs to one dequantiser group");
 };
 
 struct TcParams {
