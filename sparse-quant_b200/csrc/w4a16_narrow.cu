@@ -137,6 +137,10 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
         mbar_arrive_expect_tx(bar, 8192);
         tma_load_2d(dst, &w_map, nb * 256, ks * 4, bar);
     };
+    // Under programmatic launch the previous grid may still run for as long as it likes (a fused exchange waits seconds for a
+    // peer): whoever waits, directly or through others, for something the activations set off does so only behind this, or the
+    // bounded waits would count the previous grid's time as their own and give up.
+    auto after_previous = [&]() { if (p.pdl) asm volatile("griddepcontrol.wait;" ::: "memory"); };
     constexpr int kEarly = 2;                                        // stages requested before the rest of the CTA is set up
     if (warp == 0) {
         if (lane < Q) {
@@ -165,6 +169,7 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
         int st = 0, nb = nb0, ks = ks0; uint32_t phase = 0;
         bool ok = true;
         for (int it = 0; it < total; ++it) {
+            if (it == Q) after_previous();
             if (it >= Q && !(ok = __all_sync(0xffffffffu, mbar_wait(wempty_bar(st), phase ^ 1u, abort_flag, kWaitBudgetNs)))) break;
             if ((it >= kEarly || it >= ks1 - ks0) && elect_one()) load_weights(st, nb, ks);
             __syncwarp();
@@ -177,7 +182,7 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
         }
     } else if (warp == 1) {
         // ---- activations ----
-        if (p.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
+        after_previous();
         int st = 0, ks = ks0; uint32_t phase = 0;
         bool ok = true;
         for (int it = 0; it < total; ++it) {
@@ -199,6 +204,7 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
         int st = 0, nb = nb0, ks = ks0; uint32_t phase = 0;
         bool ok = true;
         for (int it = 0; it < total; ++it) {
+            if (it == Q) after_previous();
             if (it >= Q && !(ok = __all_sync(0xffffffffu, mbar_wait(wempty_bar(st), phase ^ 1u, abort_flag, kWaitBudgetNs)))) break;
             if (elect_one()) {
                 mbar_arrive_expect_tx(wfull_bar(st), GPS * 512);
@@ -224,6 +230,7 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
             if (++ahead == Q) { ahead = 0; ahead_phase ^= 1u; }
             return r;
         };
+        after_previous();
         ready0 = probe();
         ready1 = probe();
         for (int it = 0; it < total; ++it) {
@@ -265,7 +272,9 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
                 const bool turned = !(shallow && it >= Q) || mbar_test_wait(done_bar(st), phase ^ 1u);
                 bool loaded = mbar_test_wait(wfull_bar(st), phase);                  // the probes are in flight together
                 const bool slot_free = it < R || mbar_test_wait(done_bar(freed), freed_phase);
+                const bool first = it >= R && it < R + kDequantSets;                 // this set's first wait for an MMA
                 if (!__all_sync(0xffffffffu, turned)) {
+                    if (first) after_previous();
                     if (!__all_sync(0xffffffffu, mbar_wait(done_bar(st), phase ^ 1u, abort_flag, kWaitBudgetNs))) break;
                     loaded = false;                                                  // asked before that round was known to be over
                 }
@@ -287,6 +296,7 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
                     }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(wempty_bar(st));
+                if (first) after_previous();
                 if (!slot_free && !mbar_wait(done_bar(freed), freed_phase, abort_flag, kWaitBudgetNs)) break;
                 __syncwarp();
                 tc_fence_after_sync();
@@ -351,6 +361,7 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
         float acc[EC];
 #pragma unroll
         for (int i = 0; i < EC; ++i) acc[i] = 0.f;
+        after_previous();
         float* red = reinterpret_cast<float*>(smem + red_off) + col0 * kBlockN + quarter * 32 + lane;
         for (int base = 0; base < total && ok; base += kAhead) {
             // unrolled over the scales in flight: handing them down a register queue would wait for the newest load
@@ -407,7 +418,7 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
     }
     cg::cluster_group cluster = cg::this_cluster();
     if (S > 1) cluster.sync();
-    if (p.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");    // outputs and residual belong to earlier work until then
+    after_previous();                                                // outputs and residual belong to earlier work until then
     auto total_of = [&](int blk, int tok, int f) {
         const uint32_t at = red_base + (uint32_t)(blk * Cfg::kRedBytes + (tok * kBlockN + f) * 4);
         float v[8];

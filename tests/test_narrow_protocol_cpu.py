@@ -57,24 +57,35 @@ class Bar:
         return (self.phase & 1) != parity
 
 
-def simulate(Q, R, DR, total, seed, guarded):
-    """-> list of (role, stage) whose wait passed a round early, plus ('overrun', name) for barriers hit too often."""
+def simulate(Q, R, DR, total, seed, guarded, previous_ends=0, held=lambda role: True):
+    """-> list of (role, stage) whose wait passed a round early, plus ('overrun', name) for barriers hit too often and
+    ('counts the previous grid', role, stage) for waits that were already running when the previous grid of a programmatic
+    launch ended; `held` says which roles wait for that grid before they wait for anything the activations set off."""
     rng = random.Random(seed)
     ready, done = [Bar(3) for _ in range(Q)], [Bar(1) for _ in range(Q)]
     wfull, wempty = [Bar(2) for _ in range(Q)], [Bar(1) for _ in range(Q)]
-    early, landing = [], []
+    early, landing, now = [], [], [0]
 
     def wait(role, bars, it):                                     # wait for the round of stage `it` (it < 0: passes at once)
+        since = now[0]
         while not bars[it % Q].passes((it // Q) & 1):
             yield 1
+        if since < previous_ends <= now[0] and bars is not wfull:
+            early.append(("counts the previous grid", role, it))
         if bars[it % Q].phase < it // Q + 1:
             early.append((role, it))
 
     def latency():
         return rng.choice((20, 25, 30)) if rng.random() < 0.85 else rng.randrange(100, 600)
 
+    def after_previous(role):
+        while held(role) and now[0] < previous_ends:
+            yield 1
+
     def weights(role):
         for it in range(total):
+            if it == Q:
+                yield from after_previous("weights")
             if it >= Q:
                 yield from wait(role, wempty, it - Q)
             wfull[it % Q].arrive(1)
@@ -82,6 +93,8 @@ def simulate(Q, R, DR, total, seed, guarded):
             yield 2
 
     def activations():
+        while now[0] < previous_ends:
+            yield 1
         for it in range(total):
             if it >= Q:
                 yield from wait("x", done, it - Q)
@@ -90,6 +103,7 @@ def simulate(Q, R, DR, total, seed, guarded):
             yield 2
 
     def mma():
+        yield from after_previous("MMA")
         for it in range(total):
             yield from wait("mma", ready, it)
             yield 4
@@ -97,11 +111,15 @@ def simulate(Q, R, DR, total, seed, guarded):
 
     def dequantiser(s):
         for it in range(s, total, SETS):
+            if R <= it < R + SETS and guarded(Q, R) and it >= Q:
+                yield from after_previous("dequantisers")
             if guarded(Q, R) and it >= Q:
                 yield from wait("dequantiser, stage before", done, it - Q)
             yield from wait("dequantiser", wfull, it)
             yield 2
             wempty[it % Q].arrive()
+            if R <= it < R + SETS:
+                yield from after_previous("dequantisers")
             if it >= R:
                 yield from wait("dequantiser, A slot", done, it - R)
             yield 6
@@ -110,6 +128,7 @@ def simulate(Q, R, DR, total, seed, guarded):
     def epilogue():
         for it in range(min(DR, total)):
             ready[it % Q].arrive()
+        yield from after_previous("scale and accumulate")
         for it in range(total):
             yield from wait("epilogue", done, it)
             yield 3
@@ -117,7 +136,7 @@ def simulate(Q, R, DR, total, seed, guarded):
                 ready[(it + DR) % Q].arrive()
 
     procs = [[0, p] for p in (weights("w"), weights("zs"), activations(), mma(), epilogue())] + [[0, dequantiser(s)] for s in range(SETS)]
-    for _ in range(400 * total):
+    for now[0] in range(400 * total + previous_ends):
         for c in landing:
             c[0] -= 1
             if c[0] == 0:
@@ -165,3 +184,21 @@ def test_the_model_sees_the_early_pass_of_a_shallow_ring_without_the_wait():
         return any(simulate(q, r, dr, 5 * q + 3, seed, lambda *_: False) for seed in range(40))
     assert found(5, 4, 4) and found(6, 4, 2) and found(7, 4, 4)   # every depth the 64-token tile has
     assert not found(8, 4, 4) and not found(10, 6, 4)             # from R + 4 on a set's own history vouches for it
+
+
+def _role(name):
+    """The kernel's source from the role's headline to the next one."""
+    return SOURCE.split("// ---- " + name)[1].split("// ---- ")[0]
+
+
+def test_waits_behind_the_previous_grid_do_not_count_its_time():
+    """Programmatic launch: the activations arrive when the previous grid has ended, however late.  Nobody may be inside a
+    bounded wait for something they set off by then (the weights' own barriers are filled before)."""
+    def kernel(role):
+        names = {"weights": ("packed weights", "(zero, scale) rows"), "MMA": ("MMA",), "dequantisers": ("dequantisers",),
+                 "scale and accumulate": ("scale and accumulate",)}[role]
+        return all("after_previous()" in _role(n) for n in names)
+
+    for q, r, dr in sorted({rings(T, G, b) for T, G, b in SHAPES if T < 64}):
+        assert simulate(q, r, dr, 4 * q, 1, kernel_guards, previous_ends=600, held=kernel) == [], (q, r, dr)
+    assert any("counts the previous grid" in e for e in simulate(10, 6, 4, 40, 1, kernel_guards, previous_ends=600, held=lambda role: False))
