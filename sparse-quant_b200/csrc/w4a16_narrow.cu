@@ -141,6 +141,10 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
     // peer): whoever waits, directly or through others, for something the activations set off does so only behind this, or the
     // bounded waits would count the previous grid's time as their own and give up.
     auto after_previous = [&]() { if (p.pdl) asm volatile("griddepcontrol.wait;" ::: "memory"); };
+    // Waits that can fail are decided by the whole warp: lanes probe, read the timer and the abort flag one by one, and a warp
+    // that parted here would run into the warp-wide instructions behind the wait in pieces.
+    auto all = [](bool b) { return __all_sync(0xffffffffu, b) != 0; };
+    auto wait_all = [&](uint32_t bar, uint32_t parity) { return all(mbar_wait(bar, parity, abort_flag, kWaitBudgetNs)); };
     constexpr int kEarly = 2;                                        // stages requested before the rest of the CTA is set up
     if (warp == 0) {
         if (lane < Q) {
@@ -170,7 +174,7 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
         bool ok = true;
         for (int it = 0; it < total; ++it) {
             if (it == Q) after_previous();
-            if (it >= Q && !(ok = __all_sync(0xffffffffu, mbar_wait(wempty_bar(st), phase ^ 1u, abort_flag, kWaitBudgetNs)))) break;
+            if (it >= Q && !(ok = wait_all(wempty_bar(st), phase ^ 1u))) break;
             if ((it >= kEarly || it >= ks1 - ks0) && elect_one()) load_weights(st, nb, ks);
             __syncwarp();
             if (++ks == ks1) { ks = ks0; ++nb; }
@@ -186,7 +190,7 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
         int st = 0, ks = ks0; uint32_t phase = 0;
         bool ok = true;
         for (int it = 0; it < total; ++it) {
-            if (it >= Q && !(ok = __all_sync(0xffffffffu, mbar_wait(done_bar(st), phase ^ 1u, abort_flag, kWaitBudgetNs)))) break;
+            if (it >= Q && !(ok = wait_all(done_bar(st), phase ^ 1u))) break;
             if (elect_one()) {
                 mbar_arrive_expect_tx(ready_bar(st), Cfg::kXStage);
                 tma_load_3d(smem_base + st * Cfg::kXStage, &x_map, 0, 0, 2 * ks, ready_bar(st));
@@ -205,7 +209,7 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
         bool ok = true;
         for (int it = 0; it < total; ++it) {
             if (it == Q) after_previous();
-            if (it >= Q && !(ok = __all_sync(0xffffffffu, mbar_wait(wempty_bar(st), phase ^ 1u, abort_flag, kWaitBudgetNs)))) break;
+            if (it >= Q && !(ok = wait_all(wempty_bar(st), phase ^ 1u))) break;
             if (elect_one()) {
                 mbar_arrive_expect_tx(wfull_bar(st), GPS * 512);
                 tma_load_2d(smem_base + w_off + st * Cfg::kWStage + 8192, &zs_map, nb * kBlockN, ks * GPS, wfull_bar(st));
@@ -234,8 +238,7 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
         ready0 = probe();
         ready1 = probe();
         for (int it = 0; it < total; ++it) {
-            if (!ready0 && !mbar_wait(ready_bar(st), phase, abort_flag, kWaitBudgetNs)) break;     // the same for every lane
-            __syncwarp();
+            if (!all(ready0) && !wait_all(ready_bar(st), phase)) break;
             tc_fence_after_sync();
             const bool ready2 = probe();
             const uint64_t bdesc = bdesc0 + (uint64_t)((uint32_t)(st * Cfg::kXStage) >> 4);
@@ -273,13 +276,12 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
                 bool loaded = mbar_test_wait(wfull_bar(st), phase);                  // the probes are in flight together
                 const bool slot_free = it < R || mbar_test_wait(done_bar(freed), freed_phase);
                 const bool first = it >= R && it < R + kDequantSets;                 // this set's first wait for an MMA
-                if (!__all_sync(0xffffffffu, turned)) {
+                if (!all(turned)) {
                     if (first) after_previous();
-                    if (!__all_sync(0xffffffffu, mbar_wait(done_bar(st), phase ^ 1u, abort_flag, kWaitBudgetNs))) break;
+                    if (!wait_all(done_bar(st), phase ^ 1u)) break;
                     loaded = false;                                                  // asked before that round was known to be over
                 }
-                if (!loaded && !mbar_wait(wfull_bar(st), phase, abort_flag, kWaitBudgetNs)) break;    // the same for every lane
-                __syncwarp();
+                if (!all(loaded) && !wait_all(wfull_bar(st), phase)) break;
                 const unsigned char* wst = smem + w_off + st * Cfg::kWStage;
                 const uint4* wq = reinterpret_cast<const uint4*>(wst) + quarter * 32 + lane;
                 const uint32_t* zsp = reinterpret_cast<const uint32_t*>(wst + 8192) + quarter * 32 + (lane >> 2);
@@ -297,8 +299,7 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
                 __syncwarp();
                 if (lane == 0) mbar_arrive(wempty_bar(st));
                 if (first) after_previous();
-                if (!slot_free && !mbar_wait(done_bar(freed), freed_phase, abort_flag, kWaitBudgetNs)) break;
-                __syncwarp();
+                if (!all(slot_free) && !wait_all(done_bar(freed), freed_phase)) break;
                 tc_fence_after_sync();
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
@@ -369,7 +370,7 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
             for (int u = 0; u < kAhead; ++u) {
                 const int it = base + u;
                 if (it >= total) break;
-                ok = __all_sync(0xffffffffu, mbar_wait(done_bar(st), phase, abort_flag, kWaitBudgetNs));
+                ok = wait_all(done_bar(st), phase);
                 if (!ok) break;
                 tc_fence_after_sync();
                 float s0[GPS];
