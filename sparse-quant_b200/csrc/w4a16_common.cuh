@@ -227,5 +227,6 @@ int launch_tc(const GemmArgs& a, void* workspace, size_t workspace_bytes, cudaSt
               int force_split = 0);
 size_t tc_workspace_bytes(int tokens, int N, int K, int g);
 bool tc_supported(int tokens, int N, int K, int g);
+double tc_small_time_ns(int tokens, int N, int K);
 
 }  // namespace w4a16

@@ -611,16 +611,32 @@ bool narrow_supported(int tokens, int N, int K, int g)
     return tokens > 0 && tokens <= 64 && (g == 64 || g == 128) && (K % 64) == 0 && (N % kTileN) == 0;
 }
 
+// Time of a call of 33 to 64 tokens in ns, fitted to graphs of calls on weights from HBM (138 shapes, 768 <= K <= 16384,
+// 768 <= N <= 22016, both group sizes, 33, 48 and 64 tokens: within 18 %).
+template <int G>
+static double narrow_time_ns(int tokens, int N, int K)
+{
+    const NarrowPlan pl = plan_narrow<64, G>(N, K);
+    if (pl.blocks == 0) return 1e30;
+    const int k_steps = (K + kBlockK - 1) / kBlockK, stages = pl.blocks * ((k_steps + pl.splits - 1) / pl.splits);
+    return 5400.0 + stages * (G == 64 ? 680.0 : 460.0) + 1800.0 * pl.blocks - (pl.splits > 1 ? 1400.0 : 0.0) + 38.0 * (tokens - 32);
+}
+
 bool narrow_preferred(int tokens, int N, int K, int g)
 {
     // Measured in graphs of calls on weights from HBM, us, mma.sync kernels / this one: at 32 tokens 12.8 / 8.5 (4096 -> 4096),
     // 23.9 / 15.8 (12288), 26.3 / 17.6 (16384), 32.3 / 17.8 (16384 -> 4096), 35.4 / 28.4 (4096 -> 22016, g = 64): from 17 on.
     // At 9 to 16 tokens they are level with groups of 128 (7.4 / 7.8, 14.9 / 14.1, 15.4 / 15.6, 16.6 / 16.6), this one
-    // ahead with groups of 64, twice the scale work for them (29.6 / 23.3, 15.8 / 13.5).  At 33 to 64 the prefill kernel's
-    // 64-token tile, which does not split a short K, leaves SMs idle on all but the widest matrices: at 48 tokens 16.3 / 9.3
-    // (4096 -> 4096), 26.7 / 20.0 (11008 -> 4096), 30.3 / 20.0 (16384 -> 4096), but 17.1 / 20.3 (4096 -> 12288), 31.2 / 41.2 (22016).
+    // ahead with groups of 64, twice the scale work for them (29.6 / 23.3, 15.8 / 13.5; of 138 shapes the mma.sync kernels
+    // were ahead by more than 3 % on six, all with K <= 2048 and 4096 <= N <= 9600, at most 5.6 / 6.3).
+    // At 33 to 64 the prefill kernel's 64-token tile takes one CTA per out-feature block and leaves SMs idle on narrow
+    // matrices, where this one splits K; on wide ones this one takes several blocks per cluster, on shallow rings, and its
+    // share per stage is larger, with groups of 64 above all.  Prefill kernel / this one at 48 tokens: 17.0 / 10.2
+    // (4096 -> 4096), 17.4 / 14.9 (9472), 17.6 / 18.2 (11008), 17.8 / 22.1 (12288); with g = 64 16.9 / 12.0, 17.5 / 18.1,
+    // 17.6 / 22.8, 17.7 / 29.4; short K 7.5 / 8.0 (768 -> 4096, g = 64), 8.3 / 11.8 (11008).  So their times are compared;
+    // over the 414 measured points the choice loses 0.3 % to the better one on average, 3 to 10 % on fourteen.
     if (!narrow_supported(tokens, N, K, g)) return false;
-    if (tokens > 32) return N < 12288;
+    if (tokens > 32) return (g == 64 ? narrow_time_ns<64>(tokens, N, K) : narrow_time_ns<128>(tokens, N, K)) < tc_small_time_ns(tokens, N, K);
     return tokens > (g == 64 ? 8 : 16);
 }
 

@@ -416,3 +416,31 @@ def test_narrow_is_no_less_exact_than_the_decode_kernels_and_keeps_their_epilogu
         ref = x[0].double() @ w.reshape(N, K).t()
         err = {k: ((o - ref).norm() / ref.norm()).item() for k, o in outs.items()}
         assert err[3] <= 1.02 * err[1] and err[3] <= 2.0 ** -11, err       # an fp16 rounding is at most 2^-11 of each output
+
+
+@pytest.mark.parametrize("M,N,K,g,kernel", [
+    (8, 512, 1024, 64, "decode"), (9, 512, 1024, 64, "batched"), (16, 512, 1024, 128, "decode"), (17, 512, 1024, 128, "batched"),
+    (32, 512, 1024, 64, "batched"), (33, 512, 1024, 64, "batched"), (64, 512, 2048, 128, "batched"), (65, 512, 1024, 64, "prefill"),
+    # 33 to 64 tokens go to the kernel that is faster there: wide matrices and a short K with groups of 64 to the prefill kernel
+    (48, 4096, 2048, 128, "batched"), (33, 9472, 4096, 128, "batched"), (48, 11008, 1024, 64, "prefill"), (48, 11008, 4096, 64, "prefill"),
+    (64, 9600, 768, 128, "prefill"), (40, 12256, 1024, 128, "prefill"), (64, 4096, 768, 64, "prefill")])
+def test_automatic_dispatch_at_its_edges(M, N, K, g, kernel):
+    """Which kernel a plain call takes (they round differently: the one forced gives the same bits), and its result."""
+    import quant
+    lib = quant.load_library()
+    p = packed(N, K, g)
+    qw, zs = to_dev(p)
+    x = make_x(M, K).cuda()
+    auto = quant.gemm_awq_bias(x, qw, zs, None, N, g)
+    forced = {}
+    try:
+        if M <= 64:
+            lib.w4a16_tune_decode(3, 0, 0, 0)
+            forced["batched"] = quant.gemm_awq_bias(x, qw, zs, None, N, g)
+    finally:
+        lib.w4a16_tune_decode(0, 0, 0, 0)
+    forced["decode" if M <= 32 else "prefill"] = quant.gemm_awq_bias(x, qw, zs, None, N, g, algo=quant.ALGO_SKINNY if M <= 32 else quant.ALGO_TC)
+    same = [k for k, v in forced.items() if torch.equal(v, auto)]
+    assert same == [kernel], same
+    if N * K <= 4096 * 2048:
+        run(M, N, K, g, algo=0, bias=True)
