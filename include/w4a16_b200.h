@@ -86,8 +86,9 @@ int w4a16_gemm_algo(const void* x, const void* qweight, const void* zeros_scales
  */
 #define W4A16_FLAG_STATIC_WEIGHTS 1u
 #define W4A16_FLAG_RELU 2u
-/* with W4A16_FLAG_RELU: NaN stays NaN, as under torch.relu (without it NaN becomes 0).  Prefill kernel only
- * (W4A16_ERR_BAD_ALGO where another kernel runs). */
+/* with W4A16_FLAG_RELU: NaN stays NaN, as under torch.relu (without it NaN becomes 0).  Prefill kernel only: beyond 32
+ * tokens W4A16_ALGO_AUTO takes that kernel for such a call; up to 32 tokens, with groups of 32 and with
+ * W4A16_ALGO_SKINNY it is W4A16_ERR_BAD_ALGO. */
 #define W4A16_FLAG_RELU_KEEPS_NAN 8u
 int w4a16_gemm_ex(const void* x, const void* qweight, const void* zeros_scales, const void* bias,
                   void* out, int tokens, int N, int K, int group_size,

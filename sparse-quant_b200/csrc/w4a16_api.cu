@@ -198,8 +198,10 @@ extern "C" int w4a16_gemm_fused(const void* x, const void* qweight, const void* 
     a.relu_keeps_nan = (flags & W4A16_FLAG_RELU_KEEPS_NAN) != 0;
 
     const int forced = decode_forced_kernel();
+    // (beyond 32 tokens a ReLU that keeps NaN takes the prefill kernel, whichever of the two the shape would get without it)
     const bool narrow = forced == 3 ? algo != W4A16_ALGO_TC && narrow_supported(tokens, N, K, group_size)
-                                    : forced == 0 && algo == W4A16_ALGO_AUTO && narrow_preferred(tokens, N, K, group_size);
+                                    : forced == 0 && algo == W4A16_ALGO_AUTO && !(a.relu_keeps_nan && tokens > 32) &&
+                                      narrow_preferred(tokens, N, K, group_size);
     if (algo == W4A16_ALGO_AUTO) algo = (tokens <= 32 || !tc_supported(tokens, N, K, group_size)) ? W4A16_ALGO_SKINNY : W4A16_ALGO_TC;
     if (a.silu_mul) {
         // the SwiGLU epilogue lives in the decode kernels (one pass of at most 32 tokens); larger inputs use

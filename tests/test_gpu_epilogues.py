@@ -206,3 +206,18 @@ def test_relu_epilogue_can_keep_nan():
         assert bool(kept[0, 3].isnan().all()) and not bool(quant.gemm_awq_bias(x, qw, zs, None, N, g, algo=quant.ALGO_TC, relu=True).isnan().any())
     with pytest.raises(RuntimeError):
         quant.gemm_awq_bias(x[:, :20].contiguous(), qw, zs, None, N, g, relu=quant.RELU_KEEPS_NAN)
+
+
+@pytest.mark.parametrize("M,N", [(33, 512), (48, 4096), (48, 12288), (64, 512)])
+def test_relu_that_keeps_nan_does_not_depend_on_which_kernel_the_shape_would_get(M, N):
+    """33 to 64 tokens: some widths go to the batched-decode kernel, which has no such ReLU; the flag takes them to the prefill kernel."""
+    import quant
+    K, g = 1024, 128
+    p = make_packed(N, K, g, seed=5)
+    qw, zs = to_dev(p)
+    x = make_x(M, K, seed=2)
+    x[0, 3, 7] = float("nan")
+    x = x.cuda()
+    kept = quant.gemm_awq_bias(x, qw, zs, None, N, g, relu=quant.RELU_KEEPS_NAN)
+    plain = torch.relu(quant.gemm_awq_bias(x, qw, zs, None, N, g, algo=quant.ALGO_TC))
+    assert torch.equal(torch.nan_to_num(kept, nan=-1.0), torch.nan_to_num(plain, nan=-1.0)) and bool(kept[0, 3].isnan().all())
