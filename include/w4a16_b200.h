@@ -105,7 +105,8 @@ int w4a16_gemm_ex(const void* x, const void* qweight, const void* zeros_scales, 
  *     out-feature tiles alternating (tile 2j = gate tile j, tile 2j+1 = up tile j; w4a16.tp.fuse_gate_up builds it in
  *     the packed domain); out is fp16 [tokens, N/2], out[t, j] = fp16(silu(gate[t, j])) * up[t, j] with gate and up
  *     rounded to fp16 (+ bias) first, i.e. the roundings of act_fn(gate_proj(x)) * up_proj(x).  Decode kernels only
- *     (tokens <= 32, N % 64 == 0, no residual); W4A16_ERR_BAD_ALGO otherwise - use w4a16_silu_mul on the plain output.
+ *     (tokens <= 32, N % 64 == 0, no residual); W4A16_ERR_BAD_ALGO otherwise - use
+ *     w4a16_silu_mul_tiles on the plain output, whose tiles alternate (w4a16_silu_mul expects all gates, then all ups).
  */
 #define W4A16_FLAG_SILU_MUL 4u
 int w4a16_gemm_fused(const void* x, const void* qweight, const void* zeros_scales, const void* bias,

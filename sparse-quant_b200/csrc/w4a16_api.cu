@@ -205,7 +205,7 @@ extern "C" int w4a16_gemm_fused(const void* x, const void* qweight, const void* 
     if (algo == W4A16_ALGO_AUTO) algo = (tokens <= 32 || !tc_supported(tokens, N, K, group_size)) ? W4A16_ALGO_SKINNY : W4A16_ALGO_TC;
     if (a.silu_mul) {
         // the SwiGLU epilogue lives in the decode kernels (one pass of at most 32 tokens); larger inputs use
-        // w4a16_silu_mul on the plain output
+        // w4a16_silu_mul_tiles on the plain output
         if (algo != W4A16_ALGO_SKINNY || tokens > 32 || (N % 64) || residual) return W4A16_ERR_BAD_ALGO;
     }
     if (a.relu_keeps_nan && (narrow || algo != W4A16_ALGO_TC)) return W4A16_ERR_BAD_ALGO;

@@ -67,3 +67,11 @@ def test_python_shim_rejects_like_the_reference():
         quant.dequant(W, ZS, 64, 128, 128)
     with pytest.raises(RuntimeError):
         quant.transpose_merge_zeros_scales(ZS, ZS, ZS, 128, 64, 128)
+
+
+def test_header_names_the_product_that_fits_the_alternating_tiles():
+    """W4A16_FLAG_SILU_MUL asks for alternating gate and up tiles; beyond its 32 tokens the product on the plain output is
+    w4a16_silu_mul_tiles - w4a16_silu_mul reads another layout and would give wrong values without an error."""
+    text = open(os.path.join(ROOT, "include", "w4a16_b200.h")).read()
+    about = " ".join(text[:text.index("int w4a16_gemm_fused(")].split("/*")[-1].split())
+    assert "W4A16_FLAG_SILU_MUL" in about and "use * w4a16_silu_mul_tiles on the plain output" in about
