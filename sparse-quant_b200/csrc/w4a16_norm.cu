@@ -183,14 +183,21 @@ using namespace w4a16;
 extern "C" int w4a16_silu_mul_tiles(const void* gate_up, void* out, int rows, int n, void* stream)
 {
     if (!gate_up || !out) return W4A16_ERR_NULL_POINTER;
-    if (rows <= 0 || n <= 0 || (n % kTileN) || (long long)rows * n >= (1ll << 31)) return W4A16_ERR_BAD_SHAPE;
+    if (rows <= 0 || n <= 0 || (n % kTileN)) return W4A16_ERR_BAD_SHAPE;
     if (((uintptr_t)gate_up & 15) || ((uintptr_t)out & 15)) return W4A16_ERR_MISALIGNED;
-    const unsigned total_vec = (unsigned)rows * (unsigned)(n / 8);
-    const unsigned blocks = (total_vec + 255) / 256 < 2368 ? (total_vec + 255) / 256 : 2368;     // 16 per SM
-    silu_mul_tiles_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>((const __half*)gate_up, (__half*)out, (unsigned)n, total_vec);
-    count_launch();
-    const cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? W4A16_OK : record_cuda_error(e);
+    // a launch counts 32-bit vectors: larger products (262144 tokens x 11008) go out in slices of rows
+    const int slice = (int)(((1ll << 31) - 1) / n);
+    for (int r0 = 0; r0 < rows; r0 += slice) {
+        const unsigned total_vec = (unsigned)(rows - r0 < slice ? rows - r0 : slice) * (unsigned)(n / 8);
+        const unsigned blocks = (total_vec + 255) / 256 < 2368 ? (total_vec + 255) / 256 : 2368;     // 16 per SM
+        silu_mul_tiles_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>((const __half*)gate_up + (size_t)r0 * 2 * n,
+                                                                        (__half*)out + (size_t)r0 * n, (unsigned)n, total_vec);
+        count_launch();
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return record_cuda_error(e);
+        if (rows - r0 <= slice) break;                                 // r0 + slice could pass the range of int
+    }
+    return W4A16_OK;
 }
 
 extern "C" int w4a16_silu_mul(const void* gate_up, void* out, int rows, int n, void* stream)

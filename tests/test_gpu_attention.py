@@ -179,3 +179,13 @@ def test_silu_mul_of_alternating_tiles(rows, n):
     y = (torch.randn(1, rows, 2 * n, generator=torch.Generator().manual_seed(n)) * 3).half().cuda()
     gate, up = split_gate_up(y)
     assert torch.equal(quant.silu_mul_tiles(y), quant.silu_mul(torch.cat((gate, up), dim=-1).contiguous()))
+
+
+def test_silu_mul_of_alternating_tiles_takes_products_of_2_to_the_31():
+    """262144 tokens x 11008 and the like: rows on both sides of the slice a launch takes, and the last ones."""
+    import quant
+    n, rows = 32768, 65540                                           # rows * n just above 2^31, slices of 65535 rows
+    y = torch.empty(1, rows, 2 * n, dtype=torch.float16, device="cuda").normal_(generator=torch.Generator(device="cuda").manual_seed(1))
+    out = quant.silu_mul_tiles(y)
+    for a, b in ((0, 3), (65530, rows)):
+        assert torch.equal(out[:, a:b], quant.silu_mul_tiles(y[:, a:b].contiguous()))
