@@ -147,7 +147,7 @@ class DecoderLayer(nn.Module):
 
     def forward(self, x, pos0: int, rope=None):
         B, S, H = x.shape
-        if x.is_cuda and H <= 8192 and H % 8 == 0 and self.head_dim % 16 == 0:
+        if _kernels_apply(self, x, pos0, rope):
             return self._forward_kernels(x, pos0, rope)
         h = self.ln1(x)
         q, k, v = self.qkv_proj(h).split(self.local_heads * self.head_dim, dim=-1)
@@ -172,6 +172,49 @@ class DecoderLayer(nn.Module):
             gate, up = split_gate_up(self.gate_up_proj(h))
             x = x + self.fc2(F.silu(gate) * up)
         return x
+
+
+def _as_built(m, cls) -> bool:
+    """`m` is a module of exactly this class that nobody looks at: no hooks, no forward of its own."""
+    return type(m) is cls and not m._forward_hooks and not m._forward_pre_hooks and "forward" not in m.__dict__
+
+
+def _halves(t) -> bool:
+    return t.dtype == torch.float16 and t.is_contiguous() and t.data_ptr() % 16 == 0
+
+
+def _norm_as_built(norm, x) -> bool:
+    """Whether quant.add_norm computes what calling `norm` on rows of x would: it reads the parameters and does not call it."""
+    if not (_as_built(norm, nn.LayerNorm) and tuple(norm.normalized_shape) == (x.shape[-1],) or _as_built(norm, RMSNorm)):
+        return False
+    w, b = norm.weight, getattr(norm, "bias", None)
+    return w is not None and _halves(w) and w.numel() == x.shape[-1] and (b is None or _halves(b)) and w.device == x.device
+
+
+def _kernels_apply(layer, x, pos0: int, rope) -> bool:
+    """Whether _layer_forward_kernels stands for the op-by-op body of DecoderLayer.forward: on the GPU, with sizes the
+    kernels take, the modules it reads or hands epilogues to still the ones the layer was built with and without hooks
+    (they are not called one by one there), caches and tables in the layout the kernels write and read, no gradient."""
+    B, S, H = x.shape
+    if not (x.is_cuda and H <= 8192 and H % 8 == 0 and layer.head_dim % 16 == 0 and x.dtype == torch.float16):
+        return False
+    if torch.is_grad_enabled() and x.requires_grad:
+        return False
+    hooks = torch.nn.modules.module
+    if hooks._global_forward_hooks or hooks._global_forward_pre_hooks:
+        return False
+    m = layer._modules
+    fc1 = m.get("fc1")
+    if not (_as_built(m["qkv_proj"], WALinear) and _as_built(m["out_proj"], RowParallelWALinear) and _as_built(m["out_proj"].linear, WALinear) and
+            _as_built(m["fc2"], RowParallelWALinear) and _as_built(m["fc2"].linear, WALinear) and
+            (_as_built(m["gate_up_proj"], WALinear) if fc1 is None else _as_built(fc1, ColumnParallelWALinear) and _as_built(fc1.linear, WALinear)) and
+            _norm_as_built(m["ln1"], x) and _norm_as_built(m["ln2"], x)):
+        return False
+    k, v = layer.k_cache, layer.v_cache
+    if not (_halves(k) and _halves(v) and k.device == v.device == x.device and k.shape == v.shape == (B, layer.local_heads, k.shape[2], layer.head_dim) and
+            0 <= pos0 and pos0 + S <= k.shape[2]):
+        return False
+    return rope is None or all(_halves(t) and t.device == x.device and tuple(t.shape) == (S, layer.head_dim) for t in rope)
 
 
 def _layer_forward_kernels(self, x, pos0: int, rope=None):
@@ -201,7 +244,7 @@ def _layer_forward_kernels(self, x, pos0: int, rope=None):
     if self.cfg.kind == "opt":
         h = h.reshape(1, B * S, H)
         # (groups of 32 run in the decode kernels, whose ReLU turns NaN into 0)
-        f = self.fc1(h, relu=RELU_KEEPS_NAN) if fold and self.cfg.group_size != 32 else torch.relu(self.fc1(h))
+        f = self.fc1(h, relu=RELU_KEEPS_NAN) if fold and self.fc1.linear.group_size != 32 else torch.relu(self.fc1(h))
     else:
         f = silu_mul_tiles(self.gate_up_proj(h))
     if fold:
@@ -319,7 +362,9 @@ class Decoder(nn.Module):
             x = layer(x, self.pos, rope)
         self.pos += S
         h = x[:, -1]
-        if h.is_cuda and h.shape[-1] <= 8192 and h.shape[-1] % 8 == 0:
+        hooks = torch.nn.modules.module
+        if h.is_cuda and h.dtype == torch.float16 and h.shape[-1] <= 8192 and h.shape[-1] % 8 == 0 and \
+                _norm_as_built(self.final_norm, h) and not (hooks._global_forward_hooks or hooks._global_forward_pre_hooks):
             from quant import add_norm
             h = add_norm(h.contiguous(), None, *_norm_args(self.final_norm))[1]
         else:

@@ -121,3 +121,107 @@ def test_prefill_kernels_match_the_torch_ops(kind, B, S):
     for a, b in zip(*got):
         rel = ((a.float() - b.float()).norm() / b.float().norm()).item()
         assert rel <= 1e-2, rel                                    # fp16 stacks: one rounding in a layer travels through the rest
+
+
+def _small(kind, **kw):
+    from w4a16.models import Decoder, DecoderConfig
+    cfg = DecoderConfig(kind, layers=2, hidden=256, heads=4, ffn=512, vocab=320, group_size=64, max_positions=512, **kw)
+    return Decoder(cfg, device="cuda", seed=5).mark_static()
+
+
+def _ids(model, B, S):
+    return torch.randint(0, model.cfg.vocab, (B, S), device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))
+
+
+@pytest.mark.parametrize("kind", ["opt", "llama"])
+@pytest.mark.parametrize("S", [40, 300])
+def test_prompt_modules_that_are_watched_or_replaced_are_called(kind, S):
+    """Decoder.forward reads its normalisations' parameters and hands epilogues to its linears; hooks on them, and modules
+    of another class in their place, have to see what the layer written op by op shows them."""
+    from w4a16.models import RMSNorm
+    model = _small(kind)
+    ids = _ids(model, 1, S)
+
+    def logits():
+        model.reset(1, S + 1)
+        return model(ids).float()
+
+    plain = logits()
+    for pick in ("ln1", "ln2", "out_proj", "fc2", "fc1" if kind == "opt" else "gate_up_proj", "qkv_proj", None):
+        module = model.final_norm if pick is None else getattr(model.layers[1], pick)
+        seen = []
+        handle = module.register_forward_hook(lambda m, args, out: seen.append((args[0].detach().clone(), out.detach().clone())))
+        got = logits()
+        handle.remove()
+        assert len(seen) == 1 and ((got - plain).norm() / plain.norm()).item() <= 1e-2, pick
+        x, y = seen[0]
+        if "norm" in type(module).__name__.lower():
+            assert ((module(x) - y).abs().max() <= 1e-2 * y.abs().max())
+        else:
+            again = module(x)                                       # the linear alone: no residual, no ReLU in what the hook saw
+            assert torch.equal(again, y), pick
+
+    class Doubled(type(model.layers[0].ln1)):
+        def forward(self, x):
+            return 2 * super().forward(x)
+
+    for where, name in ((model.layers[0], "ln2"), (model, "final_norm")):
+        old = getattr(where, name)
+        new = Doubled(256, old.eps, "cuda") if isinstance(old, RMSNorm) else Doubled(256, device="cuda", dtype=torch.float16)
+        setattr(where, name, new)
+        got = logits()
+        setattr(where, name, old)
+        assert ((got - plain).norm() / plain.norm()).item() > 0.05, name
+        if name == "final_norm":
+            assert ((got - 2 * plain).norm() / plain.norm()).item() <= 2e-2
+
+
+def test_prompt_layer_keeps_the_gradient_of_its_residual_stream():
+    model = _small("opt")
+    model.reset(1, 300)
+    x = torch.randn(1, 300, 256, device="cuda").half().requires_grad_()
+    y = model.layers[0](x, 0)
+    assert y.requires_grad
+
+
+@pytest.mark.parametrize("kind", ["opt", "llama"])
+@pytest.mark.parametrize("B", [8, 24, 40])
+def test_token_step_without_folded_norms(kind, B):
+    """One token step (static position, attention kernel, residual of fc2 in the epilogue, SwiGLU in the epilogue or on
+    alternating tiles beyond 32 sequences) against the same layers written op by op in torch around the same linears."""
+    import torch.nn.functional as F
+    from w4a16.models import apply_rope
+    from w4a16.tp import split_gate_up
+    pos, D = 9, 64
+    model = _small(kind)
+    model.reset(B, 16)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    for la in model.layers:
+        la.k_cache[:, :, :pos].normal_(generator=g)
+        la.v_cache[:, :, :pos].normal_(generator=g)
+    saved = [(la.k_cache.clone(), la.v_cache.clone()) for la in model.layers]
+    x0 = torch.randn(B, 1, 256, device="cuda", generator=g).half()
+    pos_t = torch.full((1,), pos, dtype=torch.long, device="cuda")
+    x = x0
+    with torch.no_grad():
+        for la in model.layers:
+            x = la.forward_static(x, pos_t, None if kind == "opt" else (model.rope_cos, model.rope_sin))
+        y = x0
+        for la, (k, v) in zip(model.layers, saved):
+            q, kn, vn = (t.view(B, 1, 4, D).transpose(1, 2) for t in la.qkv_proj(la.ln1(y)).split(256, dim=-1))
+            if kind == "llama":
+                cos, sin = model.rope_cos[pos:pos + 1], model.rope_sin[pos:pos + 1]
+                q, kn = apply_rope(q, cos, sin), apply_rope(kn, cos, sin)
+            k[:, :, pos:pos + 1], v[:, :, pos:pos + 1] = kn, vn
+            a = F.scaled_dot_product_attention(q, k[:, :, :pos + 1], v[:, :, :pos + 1]).transpose(1, 2).reshape(B, 1, 256)
+            y = y + la.out_proj(a)
+            h = la.ln2(y)
+            if kind == "opt":
+                y = y + la.fc2(torch.relu(la.fc1(h.reshape(1, B, 256)))).reshape(B, 1, 256)
+            else:
+                gate, up = split_gate_up(la.gate_up_proj(h))
+                y = y + la.fc2(F.silu(gate) * up)
+    assert ((x.float() - y.float()).norm() / y.float().norm()).item() <= 1e-2      # fp16 layers: roundings travel through the rest
+    for la, (k, v) in zip(model.layers, saved):
+        assert ((la.k_cache.float() - k.float()).norm() / k.float().norm()).item() <= 1e-2
+        assert ((la.v_cache.float() - v.float()).norm() / v.float().norm()).item() <= 1e-2
