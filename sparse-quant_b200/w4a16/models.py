@@ -179,6 +179,11 @@ def _as_built(m, cls) -> bool:
     return type(m) is cls and not m._forward_hooks and not m._forward_pre_hooks and "forward" not in m.__dict__
 
 
+def _global_hooks() -> bool:
+    hooks = torch.nn.modules.module
+    return bool(hooks._global_forward_hooks or hooks._global_forward_pre_hooks)
+
+
 def _halves(t) -> bool:
     return t.dtype == torch.float16 and t.is_contiguous() and t.data_ptr() % 16 == 0
 
@@ -200,8 +205,7 @@ def _kernels_apply(layer, x, pos0: int, rope) -> bool:
         return False
     if torch.is_grad_enabled() and x.requires_grad:
         return False
-    hooks = torch.nn.modules.module
-    if hooks._global_forward_hooks or hooks._global_forward_pre_hooks:
+    if _global_hooks():
         return False
     m = layer._modules
     fc1 = m.get("fc1")
@@ -279,10 +283,12 @@ def _layer_forward_static(self, x, pos_t, rope, stats=None):
         a = decode_attention(qkv, self.k_cache, self.v_cache, pos_t, self.local_heads, rope=rope).view(B, 1, -1)
         x, h = add_norm(x, self.out_proj(a), *_norm_args(self.ln2))
         if self.cfg.kind == "opt":
-            return self.fc2(self.fc1(h.reshape(1, B, H), relu=True), residual=x.reshape(1, B, H)).reshape(B, 1, H)
-        if B <= 32:
-            return self.fc2(self.gate_up_proj(h, silu_mul=True), residual=x)
-        return self.fc2(silu_mul_tiles(self.gate_up_proj(h)), residual=x)
+            f = self.fc1(h.reshape(1, B, H), relu=True)
+        else:
+            f = self.gate_up_proj(h, silu_mul=True) if B <= 32 else silu_mul_tiles(self.gate_up_proj(h))
+        if not (_as_built(self.fc2, RowParallelWALinear) and _as_built(self.fc2.linear, WALinear)) or _global_hooks():
+            return x + self.fc2(f).reshape(B, 1, H)                  # somebody looks at fc2's own output
+        return self.fc2(f, residual=x.reshape(f.shape[:-1] + (H,))).reshape(B, 1, H)
     s_in, s_mid, s_out = stats
     qkv = self.qkv_proj(x, pre_norm=(*_norm_args(self.ln1), s_in)).view(B, -1)
     a = decode_attention(qkv, self.k_cache, self.v_cache, pos_t, self.local_heads, rope=rope).view(B, 1, -1)
@@ -362,9 +368,8 @@ class Decoder(nn.Module):
             x = layer(x, self.pos, rope)
         self.pos += S
         h = x[:, -1]
-        hooks = torch.nn.modules.module
         if h.is_cuda and h.dtype == torch.float16 and h.shape[-1] <= 8192 and h.shape[-1] % 8 == 0 and \
-                _norm_as_built(self.final_norm, h) and not (hooks._global_forward_hooks or hooks._global_forward_pre_hooks):
+                _norm_as_built(self.final_norm, h) and not _global_hooks():
             from quant import add_norm
             h = add_norm(h.contiguous(), None, *_norm_args(self.final_norm))[1]
         else:

@@ -225,3 +225,29 @@ def test_token_step_without_folded_norms(kind, B):
     for la, (k, v) in zip(model.layers, saved):
         assert ((la.k_cache.float() - k.float()).norm() / k.float().norm()).item() <= 1e-2
         assert ((la.v_cache.float() - v.float()).norm() / v.float().norm()).item() <= 1e-2
+
+
+@pytest.mark.parametrize("kind", ["opt", "llama"])
+def test_token_step_hands_no_residual_to_an_fc2_that_is_watched_or_replaced(kind):
+    model = _small(kind)
+    B, pos_t = 8, torch.full((1,), 3, dtype=torch.long, device="cuda")
+    x = torch.randn(B, 1, 256, device="cuda", generator=torch.Generator(device="cuda").manual_seed(4)).half()
+    la = model.layers[0]
+
+    def step():
+        model.reset(B, 16)
+        with torch.no_grad():
+            return la.forward_static(x, pos_t, None if kind == "opt" else (model.rope_cos, model.rope_sin)).float()
+
+    plain, seen = step(), []
+    handle = la.fc2.register_forward_hook(lambda m, args, out: seen.append((args[0].clone(), out.clone())))
+    assert ((step() - plain).norm() / plain.norm()).item() <= 1e-3
+    handle.remove()
+    assert torch.equal(la.fc2(seen[0][0]), seen[0][1])
+
+    class Nothing(torch.nn.Module):
+        def forward(self, f):
+            return torch.zeros(f.shape[:-1] + (256,), dtype=f.dtype, device=f.device)
+
+    la.fc2 = Nothing()
+    assert not torch.equal(step(), plain)
