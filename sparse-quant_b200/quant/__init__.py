@@ -129,7 +129,9 @@ def _half_like(t, device: int, numel: int) -> bool:
 
 
 def _relu_flags(relu) -> int:
-    return 0 if not relu else FLAG_RELU | FLAG_RELU_KEEPS_NAN if relu == RELU_KEEPS_NAN else FLAG_RELU
+    if isinstance(relu, str) and relu == RELU_KEEPS_NAN:
+        return FLAG_RELU | FLAG_RELU_KEEPS_NAN
+    return FLAG_RELU if relu else 0
 
 
 def _plain_call(I, W, ZS, bias, N, g, residual):
@@ -170,7 +172,8 @@ FLAG_STATIC_WEIGHTS = 1
 FLAG_RELU = 2
 FLAG_SILU_MUL = 4
 FLAG_RELU_KEEPS_NAN = 8
-RELU_KEEPS_NAN = 2        # relu=RELU_KEEPS_NAN: torch.relu's treatment of NaN (prefill kernel only)
+RELU_KEEPS_NAN = "keeps NaN"        # relu=RELU_KEEPS_NAN: torch.relu's treatment of NaN (prefill kernel only); not a number,
+                                    # so that any other true value (2, a numpy bool) means the plain ReLU
 
 
 def prenorm_supported(tokens: int, K: int) -> bool:

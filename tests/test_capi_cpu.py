@@ -75,3 +75,12 @@ def test_header_names_the_product_that_fits_the_alternating_tiles():
     text = open(os.path.join(ROOT, "include", "w4a16_b200.h")).read()
     about = " ".join(text[:text.index("int w4a16_gemm_fused(")].split("/*")[-1].split())
     assert "W4A16_FLAG_SILU_MUL" in about and "use * w4a16_silu_mul_tiles on the plain output" in about
+
+
+def test_relu_argument_any_truth_value_is_the_plain_relu():
+    import numpy as np
+    for on in (True, 1, 2, 8, np.bool_(True), torch.tensor(True), "yes"):
+        assert quant._relu_flags(on) == quant.FLAG_RELU
+    for off in (False, 0, None, np.bool_(False)):
+        assert quant._relu_flags(off) == 0
+    assert quant._relu_flags(quant.RELU_KEEPS_NAN) == quant.FLAG_RELU | quant.FLAG_RELU_KEEPS_NAN
