@@ -9,7 +9,7 @@
 // accumulator D[out-feature lane][token column] lives in tensor memory.
 //
 // One persistent CTA of 608 threads per SM, warp specialised (warp 4 and the last one TMA, 5 MMA, sixteen workers:
-// dequantisers and, with the 256-token tile, epilogue warps).
+// dequantisers and, with the 256-token tile, epilogue warps; 352 threads and eight workers where a CTA has one such tile).
 //
 // What set the pace of earlier versions was the ISSUE cost of the tensor-core instructions in the one thread that may
 // issue them (measured on B200 with a loop of nothing but MMAs, 148 CTAs): from a loop that a single lane enters a
@@ -46,8 +46,8 @@
 //   warp 5   MMA issuer: tcgen05.mma kind::f16 with A from tensor memory and B from the swizzled shared-memory
 //            tile, eight K=16 instructions and two commits per stage; the barriers needed next are probed before
 //            the MMAs in front of them are issued, so that in steady state no barrier round trip sits between them.
-//   epilogue (two groups of workers: 10-17 with the 256-token tile, else the first pair after their last dequant step of
-//            the tile): tcgen05.ld the accumulator, fp32 -> fp16, release it, bias add, transposed store to
+//   epilogue (two groups of workers: 10-17 with the 256-token tile and several tiles per CTA, else the first pair after
+//            their last dequant step of the tile): tcgen05.ld the accumulator, fp32 -> fp16, release it, bias add, transposed store to
 //            out[token, out-feature].
 // No cluster fan-out is used anywhere.  Every mbarrier wait is bounded; on a timeout the CTA raises an error word
 // in global memory, drains and frees its tensor memory, and returns.
@@ -67,13 +67,16 @@ namespace {
 constexpr int kBlockN   = 128;                 // out-features per CTA tile (4 packed tiles)
 constexpr int kBlockK   = 128;                 // k per pipeline stage (4 packed tiles, eight MMAs, one commit)
 constexpr int kSubK     = 64;                  // k per swizzled activation sub-tile (128 bytes of fp16)
-// Warps 4: x TMA; 5: MMA; the last one: W TMA; the other sixteen are workers in groups of four (0-3, 6-9, 10-13, 14-17).
+// Warps 4: x TMA; 5: MMA; the last one: W TMA; the others are workers in groups of four (0-3, 6-9, 10-13, 14-17).
 // Dequantiser groups: with the 256-token tile the first two (one per 64-k half of every stage), the other two being
 // epilogue warps; with the smaller tiles, whose stages are shorter than one task's latency chain, all four (taking whole
-// stages in turn), the first two draining the accumulator as well.
+// stages in turn), the first two draining the accumulator as well.  A call with at most one 256-token tile per CTA has no
+// next tile for epilogue warps of their own to hide behind and goes without them: its two groups do both, and the smaller
+// CTA starts sooner and spills no registers (us a call in graphs with four / two groups: 768 tokens 1024 -> 4096 11.4 / 10.9,
+// 1024 tokens 11.8 / 11.2, 2048 -> 4096 17.1 / 16.6, 4096 -> 4096 27.2 / 26.8).
 constexpr int kWorkerGroups = 4;
-constexpr int kWProducerWarp = 2 + 4 * kWorkerGroups;
-constexpr int kTcThreads = 32 * (kWProducerWarp + 1);
+__host__ __device__ constexpr int tc_w_producer_warp(int groups) { return 2 + 4 * groups; }
+__host__ __device__ constexpr int tc_threads(int groups) { return 32 * (tc_w_producer_warp(groups) + 1); }
 __host__ __device__ constexpr int tc_groups(int tok) { return tok == 256 ? 2 : 4; }
 constexpr int kTmemCols = 512;
 constexpr uint64_t kWaitBudgetNs = 400ull * 1000 * 1000;   // 0.4 s: far above any legitimate wait
@@ -123,8 +126,8 @@ __device__ __forceinline__ uint32_t pack_halves(uint32_t lo, uint32_t hi)
     return r;
 }
 
-template <int TOK>
-__global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map,
+template <int TOK, int WORKERS>
+__global__ void __launch_bounds__(tc_threads(WORKERS), 1) tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map,
                                                            const __grid_constant__ CUtensorMap zs_map, const TcParams p)
 {
     using Cfg = TcCfg<TOK>;
@@ -224,7 +227,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
             }
             if (!ok) drain_copies();
         }
-    } else if (warp == kWProducerWarp) {
+    } else if (warp == tc_w_producer_warp(WORKERS)) {
         // ------------------------------ TMA producer of the packed weights ------------------------------
         // One tensor copy of the stage's four k-tile rows of four packed tiles and one of its (zero, scale) rows.  (Six
         // bulk copies shared by three lanes kept this warp busy for about 900 cycles a stage: diverged lanes take turns.)
@@ -368,15 +371,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
         // packed tile column it dequantises.  With the 256-token tile group g takes the g-th 64-k half of every stage, with
         // the smaller ones every fourth stage whole: a task keeps a warp busy for a chain of dependent latencies (shared-memory load, unpack, sub/mul, tcgen05.st, its completion),
         // which the ring depth covers.  Two groups drain the accumulator (half of the columns each): with the
-        // 256-token tile groups of their own, so that the dequantisers run on into the next tile (its first stages are
-        // ready when the accumulator is free again), otherwise the first pair.
+        // 256-token tile and several tiles per CTA groups of their own, so that the dequantisers run on into the next tile
+        // (its first stages are ready when the accumulator is free again), otherwise the first pair.
         int st = 0, sw = 0; uint32_t phase = 0, wphase = 0, dphase = 0;
         bool ok = true;
         const int r = lane >> 2;
         constexpr int GROUPS = tc_groups(TOK);
-        constexpr bool kOwnEpilogue = GROUPS < kWorkerGroups;
+        constexpr bool kOwnEpilogue = GROUPS < WORKERS;
         const int quarter = warp & 3;
-        const int wgroup = warp < 4 ? 0 : (warp - 2) / 4;              // 0 .. kWorkerGroups-1
+        const int wgroup = warp < 4 ? 0 : (warp - 2) / 4;              // 0 .. WORKERS-1
         const int dgroup = wgroup & 1;                                 // which 64-k half of a stage / half of the accumulator's columns
         uint32_t step = 0;
         uint32_t epi_phase = 0;
@@ -731,7 +734,7 @@ size_t split_workspace_bytes(int tokens, int N, int split, int tiles)
     return (size_t)split * tokens * N * sizeof(float) + (((size_t)tiles * sizeof(int) + 255) / 256) * 256;
 }
 
-template <int TOK>
+template <int TOK, int WORKERS = kWorkerGroups>
 int launch_tok(const CUtensorMap& map, const CUtensorMap& w_map, const CUtensorMap& zs_map, const TcParams& p, int grid, cudaStream_t st)
 {
     static int configured[64] = {0};
@@ -739,11 +742,11 @@ int launch_tok(const CUtensorMap& map, const CUtensorMap& w_map, const CUtensorM
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return record_cuda_error(e);
     if (dev >= 64 || !configured[dev]) {
-        e = cudaFuncSetAttribute(tc_kernel<TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcCfg<TOK>::kSmemBytes);
+        e = cudaFuncSetAttribute(tc_kernel<TOK, WORKERS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcCfg<TOK>::kSmemBytes);
         if (e != cudaSuccess) return record_cuda_error(e);
         if (dev < 64) configured[dev] = 1;
     }
-    tc_kernel<TOK><<<grid, kTcThreads, TcCfg<TOK>::kSmemBytes, st>>>(map, w_map, zs_map, p);
+    tc_kernel<TOK, WORKERS><<<grid, tc_threads(WORKERS), TcCfg<TOK>::kSmemBytes, st>>>(map, w_map, zs_map, p);
     count_launch();
     e = cudaGetLastError();
     return e == cudaSuccess ? W4A16_OK : record_cuda_error(e);
@@ -840,7 +843,7 @@ int launch_tc(const GemmArgs& a, void* workspace, size_t workspace_bytes, cudaSt
     const long long items = tiles * pl.split;
     const int grid = (int)(items < sms ? items : sms);
     switch (tok) {
-        case 256: return launch_tok<256>(map, w_map, zs_map, p, grid, st);
+        case 256: return items <= sms ? launch_tok<256, 2>(map, w_map, zs_map, p, grid, st) : launch_tok<256>(map, w_map, zs_map, p, grid, st);
         case 128: return launch_tok<128>(map, w_map, zs_map, p, grid, st);
         default:  return launch_tok<64>(map, w_map, zs_map, p, grid, st);
     }

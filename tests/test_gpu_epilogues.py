@@ -221,3 +221,31 @@ def test_relu_that_keeps_nan_does_not_depend_on_which_kernel_the_shape_would_get
     kept = quant.gemm_awq_bias(x, qw, zs, None, N, g, relu=quant.RELU_KEEPS_NAN)
     plain = torch.relu(quant.gemm_awq_bias(x, qw, zs, None, N, g, algo=quant.ALGO_TC))
     assert torch.equal(torch.nan_to_num(kept, nan=-1.0), torch.nan_to_num(plain, nan=-1.0)) and bool(kept[0, 3].isnan().all())
+
+
+@pytest.mark.parametrize("M,N,K,g", [(4000, 1280, 256, 128), (256 * 13 + 1, 1504, 320, 64)])
+def test_256_token_tiles_several_per_cta(M, N, K, g):
+    """More tiles than SMs: epilogue warps of their own, half of a tile parked in tensor memory while the next one's MMAs
+    start.  Same bits as the calls of one tile per CTA (the same sums in the same order), bias, ReLU and residual as torch's
+    ops on the plain output, a ragged last tile in tokens and out-features."""
+    import quant
+    lib = quant.load_library()
+    qw, zs = to_dev(make_packed(N, K, g, seed=3))
+    x = make_x(M, K, seed=7).cuda()
+    gen = torch.Generator().manual_seed(1)
+    bias, r = torch.randn(1, N, generator=gen).half().cuda(), torch.randn(1, M, N, generator=gen).half().cuda()
+    call = lambda t, b=None, **kw: quant.gemm_awq_bias(t, qw, zs, b, N, g, algo=quant.ALGO_TC, **kw)
+    try:
+        lib.w4a16_tune_tc(256, 1)
+        plain = call(x)
+        for a in range(0, M, 1536):                                 # at most 72 tiles
+            assert torch.equal(plain[:, a:a + 1536], call(x[:, a:a + 1536].contiguous()))
+        assert torch.equal(call(x, bias), plain + bias)
+        assert torch.equal(call(x, relu=True), torch.relu(plain))
+        assert torch.equal(call(x, residual=r), plain + r)
+        assert torch.equal(call(x, bias, relu=True, residual=r), torch.relu(plain + bias) + r)
+        for a in (0, M - 300):                                      # the same epilogues with one tile per CTA
+            xs, rs = x[:, a:a + 300].contiguous(), r[:, a:a + 300].contiguous()
+            assert torch.equal(call(xs, bias, relu=True, residual=rs), (torch.relu(plain + bias) + r)[:, a:a + 300])
+    finally:
+        lib.w4a16_tune_tc(0, 0)
