@@ -444,3 +444,55 @@ def test_automatic_dispatch_at_its_edges(M, N, K, g, kernel):
     assert same == [kernel], same
     if N * K <= 4096 * 2048:
         run(M, N, K, g, algo=0, bias=True)
+
+
+@pytest.mark.parametrize("M,g", [(9, 64), (16, 64), (24, 128), (32, 128), (32, 64)])
+def test_batched_decode_in_a_dependent_chain_of_static_weights(M, g):
+    """The batched-decode kernel under programmatic launch (what a model's token step of 9 to 32 sequences runs): early weight
+    copies, waits behind the previous grid, dependents launched early.  Every call consumes the previous one's output, with
+    other kernels of the library in between; eagerly and replayed in a graph the bits are those of the plain launches."""
+    import quant
+    N = K = 1024
+    devs = [to_dev(make_packed(N, K, g, seed=50 + i)) for i in range(3)]
+    x = (make_x(M, K) * 0.5).cuda()
+    weight = torch.ones(N, dtype=torch.float16, device="cuda")
+
+    def chain(static):
+        h = x
+        for i in range(8):
+            qw, zs = devs[i % 3]
+            h = quant.gemm_awq_bias(h, qw, zs, None, N, g, static_weights=static, relu=i == 4, residual=h if i % 3 == 1 else None)
+            if i % 3 == 2:
+                h = quant.add_norm(h, None, weight, None, 1e-5, True)[1]
+        return h
+
+    plain = chain(False)
+    assert bool(plain.isfinite().all()) and float(plain.float().abs().max()) > 0
+    for _ in range(20):
+        assert torch.equal(chain(True), plain)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = chain(True)
+    for _ in range(20):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, plain)
+
+
+@pytest.mark.parametrize("M,N,K,g", [(9, 416, 1344, 64), (24, 96, 1024, 128), (32, 1376, 512, 64), (40, 416, 2048, 128), (64, 32, 1024, 64)])
+def test_batched_decode_relu(M, N, K, g):
+    """ReLU and its order with bias and residual in the batched-decode kernel, also where the last block has few out-features."""
+    import quant
+    lib = quant.load_library()
+    qw, zs = to_dev(packed(N, K, g))
+    x = make_x(M, K).cuda()
+    gen = torch.Generator().manual_seed(8)
+    b, r = torch.randn(1, N, generator=gen).half().cuda(), torch.randn(1, M, N, generator=gen).half().cuda()
+    try:
+        lib.w4a16_tune_decode(3, 0, 0, 0)
+        plain = quant.gemm_awq_bias(x, qw, zs, None, N, g)
+        assert torch.equal(quant.gemm_awq_bias(x, qw, zs, None, N, g, relu=True), torch.relu(plain))
+        assert torch.equal(quant.gemm_awq_bias(x, qw, zs, b, N, g, relu=True, residual=r), torch.relu(plain + b) + r)
+    finally:
+        lib.w4a16_tune_decode(0, 0, 0, 0)
