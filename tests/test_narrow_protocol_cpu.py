@@ -204,9 +204,17 @@ def test_waits_behind_the_previous_grid_do_not_count_its_time():
     assert any("counts the previous grid" in e for e in simulate(10, 6, 4, 40, 1, kernel_guards, previous_ends=600, held=lambda role: False))
 
 
-def test_waits_that_can_fail_are_decided_by_the_whole_warp():
-    """A bounded wait may end differently for two lanes (timer, abort flag); behind it stand warp-wide instructions."""
+def test_a_lane_that_gives_up_does_not_leave_its_warp():
+    """A bounded wait may end differently for two lanes (timer, abort flag), and behind it stand warp-wide instructions: the
+    producers vote, in the other roles no wait ends a loop and a lane that gave up neither arrives nor issues."""
     kernel = SOURCE.split("narrow_kernel(const")[1].split("int g_force_blocks")[0]
-    assert kernel.count("mbar_wait(") == 1 and "return all(mbar_wait(bar, parity, abort_flag, kWaitBudgetNs)); };" in kernel
-    for probe in ("ready0", "turned", "loaded", "slot_free"):
-        assert f"!all({probe})" in kernel and f"!{probe} " not in kernel
+    assert kernel.count("mbar_wait(") == 2                           # in the two helpers
+    for name in ("packed weights", "activations", "(zero, scale) rows"):
+        assert "wait_all(" in _role(name) and "wait_here(" not in _role(name)
+    for name in ("MMA", "dequantisers", "scale and accumulate"):
+        role = _role(name)
+        assert "wait_here(" in role and "wait_all(" not in role
+        assert role.replace("if (it >= total) break;", "").count("break") == 0
+        for line in role.splitlines():
+            if ("mbar_arrive(" in line or "elect_one()" in line) and "it < R" not in line and "i < DR" not in line:
+                assert "live" in line, line
