@@ -67,6 +67,7 @@ struct NarrowCfg {
     static constexpr int kRedBytes = T * kBlockN * 4;                    // fp32 sums of one out-feature block
     static_assert(kDCol + T * kGroups * kDRing <= 512, "tensor memory");
     static_assert(8 * kBarriers + 8 <= kBarBytes, "barrier area");
+    static bool guard(int stages) { return stages < kRing + kDequantSets; }
     static int stages(int blocks)                                        // depth of the weight and activation rings
     {
         const int room = (kNarrowSmem - 1024 - kBarBytes - blocks * kRedBytes) / (kXStage + kWStage);
@@ -105,7 +106,8 @@ __device__ __forceinline__ uint32_t sub_h2(uint32_t a, uint32_t b)
     return r;
 }
 
-template <int T, int G>
+// GUARD: the rings are so shallow that the dequantisers need the extra wait explained there (the 64-token tile's always are)
+template <int T, int G, bool GUARD>
 __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map,
                                                                            const __grid_constant__ CUtensorMap zs_map, const NarrowParams p)
 {
@@ -141,14 +143,22 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
     // peer): whoever waits, directly or through others, for something the activations set off does so only behind this, or the
     // bounded waits would count the previous grid's time as their own and give up.
     auto after_previous = [&]() { if (p.pdl) asm volatile("griddepcontrol.wait;" ::: "memory"); };
-    // A bounded wait may end differently for two lanes of a warp (they probe, read the timer and the abort flag one by one),
-    // and behind the waits stand warp-wide instructions: no lane leaves a loop on its own.  The producers, which wait for
-    // little, vote.  In the other roles a vote per wait costs 3 to 7 % of a call (32 tokens 4096 -> 22016, g = 64: 28.9 us
-    // with votes, 26.8 without): there a lane that gave up stays with its warp to the end of the loop, but waits, arrives and
-    // issues no more, so that the rest of the CTA gives up as well.
+    // Giving up.  A bounded wait may end differently for two lanes of a warp (they probe, read the timer and the flag one by
+    // one), and behind the waits stand warp-wide instructions: no lane may leave a loop on its own.  The producers vote and
+    // leave after the budget, which costs nothing.  In the other roles a vote, or a test in front of each arrival, costs 1 to 3 %
+    // of a call.  They have twice the budget: by then every producer has left or is done and no copy has been issued for as
+    // long, so an arrival too many cannot meet a barrier that only waits for bytes, and they just run their loops out.
     auto wait_all = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, kWaitBudgetNs)) != 0; };
-    bool live = true;
-    auto wait_here = [&](uint32_t bar, uint32_t parity) { if (live) live = mbar_wait(bar, parity, abort_flag, kWaitBudgetNs); };
+    auto wait_on = [&](uint32_t bar, uint32_t parity) {
+        constexpr uint32_t kProbeNs = 50000;
+        constexpr int kRunOut = 2;
+        if (mbar_try_wait(bar, parity, kProbeNs)) return;
+        const uint64_t t0 = globaltimer_ns();
+        while (!mbar_try_wait(bar, parity, kProbeNs)) {
+            if (*abort_flag == kRunOut) return;
+            if (globaltimer_ns() - t0 > 2 * kWaitBudgetNs) { *abort_flag = kRunOut; return; }
+        }
+    };
     constexpr int kEarly = 2;                                        // stages requested before the rest of the CTA is set up
     if (warp == 0) {
         if (lane < Q) {
@@ -227,13 +237,13 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
         ready0 = probe();
         ready1 = probe();
         for (int it = 0; it < total; ++it) {
-            if (!ready0) wait_here(ready_bar(st), phase);
+            if (!ready0) wait_on(ready_bar(st), phase);
             __syncwarp();
             tc_fence_after_sync();
             const bool ready2 = probe();
             const uint64_t bdesc = bdesc0 + (uint64_t)((uint32_t)(st * Cfg::kXStage) >> 4);
             const uint32_t a_tmem = tmem_base + 64 * slot, d_tmem = tmem_base + Cfg::kDCol + d * (GPS * T);
-            if (elect_one() && live) {
+            if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk)
                     mma_f16_ts(d_tmem + (GPS == 2 && kk >= 4 ? T : 0), a_tmem + 8 * kk,
@@ -252,27 +262,25 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
         const int quarter = warp & 3, set = (warp - kFirstDequantWarp) >> 2;
         const uint32_t lane_field = (uint32_t)(quarter * 32) << 16;
         auto step = [](int& i, int by, int n) { i += by; const bool wrap = i >= n; if (wrap) i -= n; return wrap; };
-        int st = set, slot = set % R, freed = set + Q - R; uint32_t phase = 0, freed_phase = 1;    // freed: the stage R back, whose A slot is taken
-        if (freed >= Q) { freed -= Q; freed_phase = 0; }
+        static_assert(kDequantSets <= R, "the first A slots are free");
+        int st = set, slot = set, freed = set + Q - R; uint32_t phase = 0, freed_phase = 1;    // freed: the stage R back, whose A slot is taken
         // A wait names a round of a ring by its parity, which is only right where the round before is known to be complete.
         // What a set knows of the weights of stage it - Q, which another set unpacked, comes from its own last stage: all
         // MMAs up to it - 4 - R have run, so the weights up to there had landed.  With fewer than R + 4 stages that does not
         // reach it - Q: a set that overtook one still waiting for its weights would take those for its own, read them half
-        // landed and hand their slot to the next copy.  There it waits for the MMAs of stage it - Q first.
-        const bool shallow = Q < R + kDequantSets;
+        // landed and hand their slot to the next copy.  There (GUARD) it waits for the MMAs of stage it - Q first.
         for (int it = set; it < total; it += kDequantSets) {
             {
-                const bool turned = !(shallow && it >= Q) || mbar_test_wait(done_bar(st), phase ^ 1u);
+                const bool turned = !(GUARD && it >= Q) || mbar_test_wait(done_bar(st), phase ^ 1u);
                 bool loaded = mbar_test_wait(wfull_bar(st), phase);                  // the probes are in flight together
                 const bool slot_free = it < R || mbar_test_wait(done_bar(freed), freed_phase);
                 const bool first = it >= R && it < R + kDequantSets;                 // this set's first wait for an MMA
                 if (!turned) {
                     if (first) after_previous();
-                    wait_here(done_bar(st), phase ^ 1u);
+                    wait_on(done_bar(st), phase ^ 1u);
                     loaded = false;                                                  // asked before that round was known to be over
                 }
-                if (!loaded) wait_here(wfull_bar(st), phase);
-                __syncwarp();
+                if (!loaded) wait_on(wfull_bar(st), phase);
                 const unsigned char* wst = smem + w_off + st * Cfg::kWStage;
                 const uint4* wq = reinterpret_cast<const uint4*>(wst) + quarter * 32 + lane;
                 const uint32_t* zsp = reinterpret_cast<const uint32_t*>(wst + 8192) + quarter * 32 + (lane >> 2);
@@ -288,9 +296,9 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
                         zz[gi][i] = __byte_perm(z, z, 0x1010);
                     }
                 __syncwarp();
-                if (lane == 0 && live) mbar_arrive(wempty_bar(st));
+                if (lane == 0) mbar_arrive(wempty_bar(st));
                 if (first) after_previous();
-                if (!slot_free) wait_here(done_bar(freed), freed_phase);
+                if (!slot_free) wait_on(done_bar(freed), freed_phase);
                 __syncwarp();
                 tc_fence_after_sync();
 #pragma unroll
@@ -319,7 +327,7 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
                 tmem_wait_st();
                 tc_fence_before_sync();
                 __syncwarp();
-                if (lane == 0 && live) mbar_arrive(ready_bar(st));
+                if (lane == 0) mbar_arrive(ready_bar(st));
             }
             if (step(st, kDequantSets, Q)) phase ^= 1u;
             step(slot, kDequantSets % R, R);
@@ -361,7 +369,7 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
             for (int u = 0; u < kAhead; ++u) {
                 const int it = base + u;
                 if (it >= total) break;
-                wait_here(done_bar(st), phase);
+                wait_on(done_bar(st), phase);
                 __syncwarp();
                 tc_fence_after_sync();
                 float s0[GPS];
@@ -384,7 +392,7 @@ __global__ void __launch_bounds__(NarrowCfg<T, G>::kThreads, 1) narrow_kernel(co
                     }
                 tc_fence_before_sync();
                 __syncwarp();
-                if (lane == 0 && live && it + DR < total) mbar_arrive(ready_bar(free_st));
+                if (lane == 0 && it + DR < total) mbar_arrive(ready_bar(free_st));
                 if (it + kAhead < total) fetch(zs[u]);
                 if (++free_st == Q) free_st = 0;
                 if (++st == Q) { st = 0; phase ^= 1u; }
@@ -471,7 +479,7 @@ int g_force_blocks = 0, g_force_splits = 0;
 
 struct NarrowPlan { int blocks, splits, stages; };
 
-template <int T, int G>
+template <int T, int G, bool GUARD>
 int prepare_instance(int* max_smem_set)
 {
     static int configured[64] = {0};       // benign race: the attribute call is idempotent
@@ -479,7 +487,7 @@ int prepare_instance(int* max_smem_set)
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return record_cuda_error(e);
     if (dev >= 64 || !configured[dev]) {
-        e = cudaFuncSetAttribute(narrow_kernel<T, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, kNarrowSmem);
+        e = cudaFuncSetAttribute(narrow_kernel<T, G, GUARD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kNarrowSmem);
         if (e != cudaSuccess) return record_cuda_error(e);
         if (dev < 64) configured[dev] = 1;
     }
@@ -494,7 +502,7 @@ int max_clusters(int sp)
     static int cache[64][9] = {};          // benign race: the query is idempotent
     int dev = 0;
     if (sp <= 1) return device_sm_count();
-    if (prepare_instance<T, G>(&dev) != W4A16_OK || dev >= 64) return 0;
+    if (prepare_instance<T, G, true>(&dev) != W4A16_OK || dev >= 64) return 0;
     if (cache[dev][sp]) return cache[dev][sp] > 0 ? cache[dev][sp] : 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(1, sp, 1);
@@ -508,7 +516,7 @@ int max_clusters(int sp)
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, narrow_kernel<T, G>, &cfg) != cudaSuccess) { n = 0; (void)cudaGetLastError(); }
+    if (cudaOccupancyMaxActiveClusters(&n, narrow_kernel<T, G, true>, &cfg) != cudaSuccess) { n = 0; (void)cudaGetLastError(); }
     cache[dev][sp] = n > 0 ? n : -1;
     return n;
 }
@@ -539,11 +547,13 @@ template <int T, int G>
 int launch_instance(const GemmArgs& a, cudaStream_t st)
 {
     using Cfg = NarrowCfg<T, G>;
-    int dev = 0;
-    int s = prepare_instance<T, G>(&dev);
-    if (s != W4A16_OK) return s;
     const NarrowPlan pl = plan_narrow<T, G>(a.N, a.K);
     if (pl.blocks == 0) return W4A16_ERR_BAD_ALGO;
+    // (with one k-step, and in other corners, the rings need no second round and no guard; the instance is chosen by depth alone)
+    const bool guard = T == 64 || Cfg::guard(pl.stages);
+    int dev = 0;
+    int s = guard ? prepare_instance<T, G, true>(&dev) : prepare_instance<T, G, T == 64>(&dev);
+    if (s != W4A16_OK) return s;
     CUtensorMap x_map, w_map, zs_map;
     {
         // as [K/64][tokens][64]: a box of two is a stage's two swizzled sub-tiles, one copy
@@ -571,8 +581,8 @@ int launch_instance(const GemmArgs& a, cudaStream_t st)
     if (!p.error) return W4A16_ERR_CUDA;
     p.tokens = a.tokens; p.N = a.N; p.K = a.K;
     p.n_blocks = (a.N + kBlockN - 1) / kBlockN; p.blocks = pl.blocks; p.splits = pl.splits; p.stages = pl.stages;
-    p.relu = a.relu ? 1 : 0; p.silu_mul = a.silu_mul ? 1 : 0; 
-    p.pdl = a.static_weights && a.tokens <= 32 ? 1 : 0;              // as before: calls of more than 32 tokens keep plain stream order
+    p.relu = a.relu ? 1 : 0; p.silu_mul = a.silu_mul ? 1 : 0;
+    p.pdl = a.static_weights && a.tokens <= 32 ? 1 : 0;              // beyond 32 tokens plain stream order, like the prefill kernel that shares the range
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((p.n_blocks + pl.blocks - 1) / pl.blocks, pl.splits, 1);
     cfg.blockDim = dim3(Cfg::kThreads);
@@ -587,7 +597,8 @@ int launch_instance(const GemmArgs& a, cudaStream_t st)
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = p.pdl ? 2 : 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, narrow_kernel<T, G>, x_map, w_map, zs_map, p);
+    const cudaError_t e = guard ? cudaLaunchKernelEx(&cfg, narrow_kernel<T, G, true>, x_map, w_map, zs_map, p)
+                                : cudaLaunchKernelEx(&cfg, narrow_kernel<T, G, T == 64>, x_map, w_map, zs_map, p);
     count_launch();
     return e == cudaSuccess ? W4A16_OK : record_cuda_error(e);
 }

@@ -168,7 +168,9 @@ def kernel_guards(Q, R):
     """What the kernel does: with rings so shallow that a set's own history does not vouch for the stage's last round, its
     dequantisers wait for that round's MMAs before they look at the weights' barrier."""
     role = SOURCE.split("---- dequantisers")[1].split("---- scale and accumulate")[0]
-    return "shallow = Q < R + kDequantSets" in role and "shallow && it >= Q" in role and "done_bar(st), phase ^ 1u" in role and Q < R + SETS
+    there = "GUARD && it >= Q" in role and "done_bar(st), phase ^ 1u" in role and \
+        "guard(int stages) { return stages < kRing + kDequantSets; }" in SOURCE and "guard = T == 64 || Cfg::guard(pl.stages)" in SOURCE
+    return there and Q < R + SETS
 
 
 @pytest.mark.parametrize("T,G", sorted({s[:2] for s in SHAPES}))
@@ -206,15 +208,14 @@ def test_waits_behind_the_previous_grid_do_not_count_its_time():
 
 def test_a_lane_that_gives_up_does_not_leave_its_warp():
     """A bounded wait may end differently for two lanes (timer, abort flag), and behind it stand warp-wide instructions: the
-    producers vote, in the other roles no wait ends a loop and a lane that gave up neither arrives nor issues."""
+    producers vote before they leave; in the other roles no wait ends a loop, and none gives up before the producers have."""
     kernel = SOURCE.split("narrow_kernel(const")[1].split("int g_force_blocks")[0]
-    assert kernel.count("mbar_wait(") == 2                           # in the two helpers
+    assert kernel.count("mbar_wait(") == 1 and "__all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, kWaitBudgetNs))" in kernel
+    waits_on = kernel.split("auto wait_on")[1].split("};")[0]
+    assert "> 2 * kWaitBudgetNs) { *abort_flag = kRunOut; return; }" in waits_on and "*abort_flag)" not in waits_on
     for name in ("packed weights", "activations", "(zero, scale) rows"):
-        assert "wait_all(" in _role(name) and "wait_here(" not in _role(name)
+        assert "wait_all(" in _role(name) and "wait_on(" not in _role(name)
     for name in ("MMA", "dequantisers", "scale and accumulate"):
         role = _role(name)
-        assert "wait_here(" in role and "wait_all(" not in role
+        assert "wait_on(" in role and "wait_all(" not in role
         assert role.replace("if (it >= total) break;", "").count("break") == 0
-        for line in role.splitlines():
-            if ("mbar_arrive(" in line or "elect_one()" in line) and "it < R" not in line and "i < DR" not in line:
-                assert "live" in line, line
