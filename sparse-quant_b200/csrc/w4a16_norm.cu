@@ -154,7 +154,8 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const __half* in, __half*
 // de-interleaving into two tensors and torch's two elementwise kernels took about 50.
 __global__ void __launch_bounds__(256) silu_mul_tiles_kernel(const __half* in, __half* out, unsigned n, unsigned total_vec)
 {
-    // as in the kernel above: a GEMV launched with programmatic stream serialization may follow, eagerly or in a graph
+    // as in the kernel above, for a linear with groups of 32 behind it: the only one beyond 32 tokens that is launched with
+    // programmatic stream serialization
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const unsigned nvec = n / 8;
