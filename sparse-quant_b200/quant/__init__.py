@@ -137,8 +137,9 @@ def _relu_flags(relu) -> int:
 def _plain_call(I, W, ZS, bias, N, g, residual):
     """Whether these are correct arguments of a plain linear on the current device: every check of gemm_awq_bias in one
     pass.  An eager call of a small linear is host time (4096 x 4096, one token: the kernel runs 5 us), and the checks
-    with their messages, the device guard and the stream object took more of it than the launch."""
-    if not (isinstance(I, torch.Tensor) and isinstance(W, torch.Tensor) and I.is_cuda and W.is_cuda and I.dim() == 3 and W.dim() == 2 and
+    with their messages, the device guard and the stream object took more of it than the launch.  (Inputs of a subclass go
+    the long way: the output is a plain tensor either way.)"""
+    if not (type(I) is torch.Tensor and isinstance(W, torch.Tensor) and I.is_cuda and W.is_cuda and I.dim() == 3 and W.dim() == 2 and
             I.dtype == torch.float16 and I.is_contiguous() and W.is_contiguous() and g > 0 and N > 0):
         return False
     b, s, K = I.shape

@@ -496,3 +496,18 @@ def test_batched_decode_relu(M, N, K, g):
         assert torch.equal(quant.gemm_awq_bias(x, qw, zs, b, N, g, relu=True, residual=r), torch.relu(plain + b) + r)
     finally:
         lib.w4a16_tune_decode(0, 0, 0, 0)
+
+
+def test_an_input_of_a_tensor_subclass_gives_a_plain_output():
+    import quant
+
+    class Tagged(torch.Tensor):
+        pass
+
+    N, K, g = 64, 256, 64
+    qw, zs = to_dev(packed(N, K, g))
+    x = make_x(3, K).cuda()
+    plain = quant.gemm_awq_bias(x, qw, zs, None, N, g)
+    for t in (x.as_subclass(Tagged), torch.nn.Parameter(x, requires_grad=False)):
+        out = quant.gemm_awq_bias(t, qw, zs, None, N, g)
+        assert type(out) is torch.Tensor and torch.equal(out, plain)
