@@ -114,7 +114,9 @@ int w4a16_gemm_fused(const void* x, const void* qweight, const void* zeros_scale
                      void* workspace, size_t workspace_bytes, void* stream, int algo, unsigned flags);
 
 /* Scratch bytes w4a16_gemm needs for this problem (0 = none).  The reference has no
- * workspace (the WorkSpace argument of Gemm_awq_pure, gemm_quant.cu:45, is unused). */
+ * workspace (the WorkSpace argument of Gemm_awq_pure, gemm_quant.cu:45, is unused).  The figure is the prefill
+ * kernel's and serves W4A16_ALGO_AUTO and W4A16_ALGO_TC alike: at 33 to 64 tokens W4A16_ALGO_AUTO may take the
+ * batched-decode kernel, which checks a workspace in the same way but does not use it. */
 size_t w4a16_workspace_bytes(int tokens, int N, int K, int group_size);
 
 /*
